@@ -78,7 +78,18 @@ struct Params {
     Tables<Real> T;
     Geom<Real> G;
     Queue<Real> pin, ein, pout, eout;    // consumed / produced queues
-    double *dose;                         // batch tally per voxel
+    // Batch tallies.  The wavefronts of a group of nslot consecutive batches run
+    // together; batch slot s of voxel ir is dose[s * slot_stride + ir] (32-bit:
+    // all slots hold at most 2^28 values, and a 64-bit product here costs the
+    // photon kernel 3% on a 64^3 slab phantom).  A deposit's
+    // slot follows from its history: floor((hist - slot_first) / per), at most
+    // nslot - 1 (the run's last batch takes the remainder), by a multiply-high
+    // (slot_m, slot_l from fast_divisor(per)); several phantoms have one such
+    // triple each (pslot).
+    double *dose;
+    unsigned slot_stride;                     // nvox
+    unsigned slot_first, slot_m, slot_last;   // slot_last = nslot - 1
+    int slot_l;
     // several phantoms in one run (Multi kernels): per-phantom geometry,
     // Philox seed and source, the phantoms' first global voxel indices
     // (nprob + 1 entries, ascending) and, for the current batch, the prefix
@@ -88,6 +99,7 @@ struct Params {
     const Source *psrc;
     const int *pvoff;
     const long long *pprefix, *pfirst;
+    const uint2 *pslot;                   // (m, l) of each phantom's histories per batch
     int nprob;
     // seed-replay adjoint: dL/dE per voxel (also weights the per-history
     // tally when set), per-history weighted deposits G_h of the replayed
@@ -129,17 +141,25 @@ constexpr double VERY_FAR = 1e30;   // egs++ veryFar (egs++/egs_functions.h:105)
 constexpr double NEAR_FACE = 1.0 / 4096.0;
 
 // ------------------------------------------------------------- tallies ----
-template <class Real>
+__device__ inline unsigned batch_slot(unsigned d, unsigned m, int l, unsigned last) {
+    return min((unsigned)fdiv((int)d, m, l), last);
+}
+// Several phantoms (Multi): the batch slot is found when a particle is fetched
+// (its phantom is known there) and kept; one phantom: it is recomputed from the
+// history at the flush, which costs no register over the step.
+template <class Real, bool Multi>
 struct Acc {
     int ir;
     uint32_t hist;
     Real e;   // deposits of one particle's visit to one voxel
+    unsigned slot;
 };
 
-template <class Real>
-__device__ inline void acc_flush(const Params<Real> &P, Acc<Real> &a) {
+template <class Real, bool Multi>
+__device__ inline void acc_flush(const Params<Real> &P, Acc<Real, Multi> &a) {
     if (a.ir >= 0 && a.e > 0) {
-        atomicAdd(P.dose + a.ir, (double)a.e);
+        const unsigned slot = Multi ? a.slot : batch_slot(a.hist - P.slot_first, P.slot_m, P.slot_l, P.slot_last);
+        atomicAdd(P.dose + (slot * P.slot_stride + (unsigned)a.ir), (double)a.e);
         if (P.hist_tally) {
             long long i = (long long)a.hist - P.hist_first;
             if (i >= 0 && i < P.hist_n) atomicAdd(P.hist_tally + i, P.wvox ? P.wvox[a.ir] * (double)a.e : (double)a.e);
@@ -148,8 +168,8 @@ __device__ inline void acc_flush(const Params<Real> &P, Acc<Real> &a) {
     a.e = 0;
     a.ir = -1;
 }
-template <class Real>
-__device__ inline void deposit(const Params<Real> &P, Acc<Real> &a, int ir, uint32_t hist, Real e) {
+template <class Real, bool Multi>
+__device__ inline void deposit(const Params<Real> &P, Acc<Real, Multi> &a, int ir, uint32_t hist, Real e) {
     if (ir < 0 || !(e > 0)) return;
     if (ir != a.ir || hist != a.hist) {
         acc_flush(P, a);
@@ -265,11 +285,15 @@ __device__ inline int phantom_of(const Params<Real> &P, int ir) {
 // Loads queue record i; in a multi-phantom run the particle's phantom (and
 // with it its Philox seed) follows from its voxel index.
 template <class Real, bool Multi>
-__device__ inline void load_particle(const Params<Real> &P, const Queue<Real> &q, unsigned i, Particle<Real> &p) {
+__device__ inline void load_particle(const Params<Real> &P, const Queue<Real> &q, unsigned i, Particle<Real> &p,
+                                     Acc<Real, Multi> &acc) {
     if (Multi) {
         int k = phantom_of(P, q.ir[i]);
         q_load(q, i, P.pseeds[k], p);
         p.pb = k;
+        acc_flush(P, acc);
+        const uint2 d = P.pslot[k];
+        acc.slot = batch_slot(p.rng.hist - (unsigned)P.pfirst[k], d.x, (int)d.y, P.slot_last);
     } else {
         q_load(q, i, P.seed, p);
         p.pb = 0;
@@ -323,9 +347,9 @@ __device__ inline void annih_at_rest(const Params<Real> &P, const Queue<Real> &q
 // Queue a new electron/positron, or -- when it is already at or below the
 // cut-off -- do its :ECUT-DISCARD: right here (deposit, and annihilation at
 // rest for a positron, on its own stream): what ELECTR would do first.
-template <class Real>
+template <class Real, bool Multi>
 __device__ inline void push_charged(const Params<Real> &P, const Queue<Real> &qe, const Queue<Real> &qp,
-                                    Particle<Real> &q, Acc<Real> &acc, unsigned long long &npush,
+                                    Particle<Real> &q, Acc<Real, Multi> &acc, unsigned long long &npush,
                                     double &edep_tot, int &err) {
     if (q.E <= P.T.ecut) {
         Real edep = q.E - (Real)RM;
@@ -483,8 +507,8 @@ __device__ inline int hfl_locate(const Geom<Real> &G, Real x, Real y, Real z) {
 // cross in proportion to the path length in each.  p.ir holds the start.
 // Returns the voxel at the end of the segments, or -1 when they leave the
 // phantom; `lost` is then the energy past that point, not deposited.
-template <class Real>
-__device__ int hfl_hinge(const Params<Real> &P, Acc<Real> &acc, const Geom<Real> &G, Particle<Real> &p,
+template <class Real, bool Multi>
+__device__ int hfl_hinge(const Params<Real> &P, Acc<Real, Multi> &acc, const Geom<Real> &G, Particle<Real> &p,
                          const Real xi0[3], const Real ui0[3], Real tv, bool ch_step, Real edep, Real &lost, int &err) {
     lost = 0;
     const int loc = p.ir;
@@ -688,7 +712,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 ? 8 : 1) k_photon
     (void)s_dummy;
     Particle<Real> p;
     PhotonState<Real> s;
-    Acc<Real> acc{-1, 0u, (Real)0};
+    Acc<Real, Multi> acc{-1, 0u, (Real)0, 0u};
     AccG<Real> ga{-1, (Real)0};
     Real Gh = 0;
     bool alive = false, exhausted = false;
@@ -722,7 +746,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 ? 8 : 1) k_photon
             if (!alive) {
                 unsigned idx = base + __popc(need & ((1u << lane) - 1u));
                 if (idx < nq) {
-                    load_particle<Real, Multi>(P, P.pin, idx, p);
+                    load_particle<Real, Multi>(P, P.pin, idx, p, acc);
                     if (Adj) Gh = hist_weight(P, p);
                     alive = true;
                     s.state = 0;
@@ -1062,7 +1086,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? 6 : 1) 
     // to the next electron queue.
     Particle<Real> lstack[LSTACK];
     int sp = 0;
-    Acc<Real> acc{-1, 0u, (Real)0};
+    Acc<Real, Multi> acc{-1, 0u, (Real)0, 0u};
     EList<Real> el;
     el.n = 0;
     // adjoint: the voxel-visit lists of suspended particles; a secondary
@@ -1118,7 +1142,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? 6 : 1) 
                 edep_part = 0;
                 unsigned idx = base + __popc(need & ((1u << lane) - 1u));
                 if (idx < nq) {
-                    load_particle<Real, Multi>(P, P.ein, idx, p);
+                    load_particle<Real, Multi>(P, P.ein, idx, p, acc);
                     if (Adj) el.n = 0;
                     alive = true;
                     s.state = 0;
@@ -1670,15 +1694,21 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? 6 : 1) 
     if (err) atomicExch(P.error + 1, 1);
 }
 
-// Batch fold: sum += d, sum2 += d*d, d = 0 (DOSXYZnrc batch statistics).
-__global__ void k_batch(double *d, double *sum, double *sum2, long long n) {
+// Batch fold of a group's slots, in batch order: sum += d, sum2 += d*d, d = 0
+// (DOSXYZnrc batch statistics).
+__global__ void k_batch(double *d, double *sum, double *sum2, long long n, int nslot) {
     long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     long long stride = (long long)gridDim.x * blockDim.x;
     for (; i < n; i += stride) {
-        double x = d[i];
-        sum[i] += x;
-        sum2[i] += x * x;
-        d[i] = 0;
+        double s = sum[i], s2 = sum2[i];
+        for (int k = 0; k < nslot; ++k) {
+            const double x = d[k * n + i];
+            s += x;
+            s2 += x * x;
+            d[k * n + i] = 0;
+        }
+        sum[i] = s;
+        sum2[i] = s2;
     }
 }
 
@@ -1897,7 +1927,7 @@ struct Engine : EngineBase {
     egsgpu_config cfg;
 
     int clear_tallies(long long nv, std::string &err) override {
-        CK(cudaMemset(d_dose.p, 0, nv * sizeof(double)));
+        CK(cudaMemset(d_dose.p, 0, nv * dose_slots * sizeof(double)));
         CK(cudaMemset(d_sum.p, 0, nv * sizeof(double)));
         CK(cudaMemset(d_sum2.p, 0, nv * sizeof(double)));
         CK(cudaMemset(d_energy.p, 0, 2 * sizeof(double)));
@@ -1922,7 +1952,7 @@ struct Engine : EngineBase {
         CK(cudaMemcpy(d_counters.p, counters8, 8 * sizeof(unsigned long long), cudaMemcpyHostToDevice));
         CK(cudaMemcpy(d_sum.p, sum, nv * sizeof(double), cudaMemcpyHostToDevice));
         CK(cudaMemcpy(d_sum2.p, sum2, nv * sizeof(double), cudaMemcpyHostToDevice));
-        CK(cudaMemset(d_dose.p, 0, nv * sizeof(double)));
+        CK(cudaMemset(d_dose.p, 0, nv * dose_slots * sizeof(double)));
         return 0;
     }
     int read_profile(double *out, std::string &err) override {
@@ -1999,6 +2029,7 @@ struct Engine : EngineBase {
     unsigned capacity = 0;
     // tallies
     DevMem d_dose, d_sum, d_sum2, d_energy, d_counters, d_error, d_hist;
+    int dose_slots = 1;   // batch slots of d_dose in use (all zero between runs)
     long long hist_first = 0, hist_n = 0;
     int sm_count = 0;
     // per-kernel device time (CUDA events on the launch stream) and launches:
@@ -2218,6 +2249,7 @@ struct Engine : EngineBase {
         G.hbt = G.bt / 2;
         G.voff = 0;
         set_divisors(G);
+        dose_slots = 1;
         CK(d_dose.alloc(nvox * sizeof(double)));
         CK(d_sum.alloc(nvox * sizeof(double)));
         CK(d_sum2.alloc(nvox * sizeof(double)));
@@ -2444,6 +2476,44 @@ struct Engine : EngineBase {
         bn = (b == nbatch - 1) ? n - b * per : per;
     }
 
+    // Batches per group: the batches of a group are transported by the same
+    // wavefronts, each into a tally slot of its own.  Every wavefront ends in a
+    // tail as long as its longest history (several ms: a charged particle's
+    // steps follow one another), so batches smaller than a wavefront are
+    // grouped until they fill one: `most` histories, a wavefront that the queues
+    // hold by the estimate the chunk autotuner starts from.  A batch that fills
+    // a wavefront by itself keeps its own.  The slots take at most 2 GiB.
+    // One GB300, 10 batches one at a time -> grouped: water30 1e4 histories
+    // 52.7 -> 7.1 ms, slab64 2e6 98.7 -> 22.7 ms, 2e5 20 MeV electrons in
+    // 128^3 voxels 814 -> 164 ms.
+    static constexpr size_t SLOT_BYTES = (size_t)2 << 30;
+    int batches_per_group(long long total, int nbatch, long long most) const {
+        const long long per = std::max<long long>(1, total / nbatch);
+        long long g = std::min<long long>(most / per, (long long)(SLOT_BYTES / ((size_t)nvox * sizeof(double))));
+        g = std::max<long long>(1, std::min<long long>(g, nbatch));
+        const long long groups = (nbatch + g - 1) / g;   // of even sizes
+        return (int)((nbatch + groups - 1) / groups);
+    }
+    // Room for `slots` batch slots; the new ones are cleared.
+    int ensure_slots(int &slots, std::string &err) {
+        if (slots <= dose_slots) return 0;
+        const size_t one = (size_t)nvox * sizeof(double), had = d_dose.n / one;
+        if ((size_t)slots > had) {
+            DevMem more;
+            if (more.alloc(one * slots) != cudaSuccess) {   // not enough memory: one batch at a time
+                cudaGetLastError();
+                slots = 1;
+                return 0;
+            }
+            CK(cudaMemcpy(more.p, d_dose.p, one * dose_slots, cudaMemcpyDeviceToDevice));
+            std::swap(more.p, d_dose.p);
+            std::swap(more.n, d_dose.n);
+        }
+        CK(cudaMemset((char *)d_dose.p + one * dose_slots, 0, one * (slots - dose_slots)));
+        dose_slots = slots;
+        return 0;
+    }
+
     template <bool Multi>
     int run_impl(const Source &S, long long first, long long n, int nbatch, uint32_t seed, cudaStream_t st,
                  std::string &err) {
@@ -2464,14 +2534,23 @@ struct Engine : EngineBase {
         // (every history owns its random-number streams).
         long long chunk = cfg.chunk;
         const bool tune = chunk <= 0;
+        const double emax = std::max(S.energy, 0.1), rec_per_hist = (S.charge == 0 ? 12.0 : 16.0) + 8.0 * emax;
+        const long long chunk0 = std::max<long long>(1024, (long long)(capacity / rec_per_hist));
         if (tune) {
-            if (tuned_chunk <= 0) {
-                double emax = std::max(S.energy, 0.1);
-                double per = (S.charge == 0 ? 12.0 : 16.0) + 8.0 * emax;
-                tuned_chunk = std::max<long long>(1024, (long long)(capacity / per));
-            }
+            if (tuned_chunk <= 0) tuned_chunk = chunk0;
             chunk = tuned_chunk;
         }
+        // Batches that run together (the adjoint's replays have one batch; a
+        // recorded graph holds one set of slot parameters, so it takes all
+        // batches in one group or each on its own).
+        long long total = n;
+        if (Multi) {
+            total = 0;
+            for (long long c : phist) total += c;
+        }
+        int group = mode ? 1 : batches_per_group(total, nbatch, tune ? chunk : std::min(chunk, chunk0));
+        if (cfg.use_graph > 0 && group < nbatch) group = 1;
+        if (int rc = ensure_slots(group, err)) return rc;
         // persistent grids, one per kernel: never more CTAs than can be
         // resident at once (the photon kernel, with fewer registers, fits more
         // CTAs per SM than the electron kernel)
@@ -2527,6 +2606,12 @@ struct Engine : EngineBase {
         P.T = T; P.G = G;
         if (hfl) P.T.etab = (const Real *)d_etab_hfl.p;
         P.dose = (double *)d_dose.p;
+        P.slot_stride = (unsigned)nvox;
+        if (!Multi && group > 1) {
+            P.slot_first = (unsigned)first;
+            fast_divisor((uint32_t)(n / nbatch), P.slot_m, P.slot_l);
+            P.slot_last = group - 1;
+        }
         P.hist_tally = (!Multi && hist_n > 0) ? (double *)d_hist.p : nullptr;
         P.hist_first = hist_first; P.hist_n = hist_n;
         P.energy = (double *)d_energy.p;
@@ -2541,7 +2626,18 @@ struct Engine : EngineBase {
             P.probs = (const Geom<Real> *)d_probs.p; P.pseeds = (const uint32_t *)d_pseeds.p;
             P.psrc = (const Source *)d_psrc.p; P.pvoff = (const int *)d_pvoff.p;
             P.pprefix = (const long long *)d_pprefix.p; P.pfirst = (const long long *)d_pfirst.p;
+            P.pslot = (const uint2 *)d_pslot.p;
             P.nprob = nprob;
+            if (group > 1) {
+                std::vector<uint2> div(nprob);
+                for (int k = 0; k < nprob; ++k) {
+                    int l;
+                    fast_divisor((uint32_t)std::max<long long>(1, phist[k] / nbatch), div[k].x, l);
+                    div[k].y = (unsigned)l;
+                }
+                CK(cudaMemcpy(d_pslot.p, div.data(), nprob * sizeof(uint2), cudaMemcpyHostToDevice));
+            }
+            P.slot_last = group - 1;
         }
         if (mode) {   // a replay for the adjoint: its own tallies, never the run's
             P.dose = mode->dose; P.energy = mode->energy; P.counters = mode->counters;
@@ -2561,14 +2657,22 @@ struct Engine : EngineBase {
         CK(cudaStreamWaitEvent(ws, ev_in, 0));
         CK(set_caps(ws));
         std::vector<long long> hprefix(nprob + 1), hfirst(nprob + 1);
-        for (int b = 0; b < nbatch; ++b) {
+        for (int b = 0; b < nbatch; b += group) {
+            const int nb = std::min(group, nbatch - b);   // batches [b, b + nb) run together
             long long b0, bn;
+            // the histories of batches [b, b + nb) of a run of cnt from f0
+            auto group_range = [&](long long f0, long long cnt, long long &f, long long &c) {
+                long long f1, c1;
+                batch_range(f0, cnt, nbatch, b, f, c);
+                batch_range(f0, cnt, nbatch, b + nb - 1, f1, c1);
+                c = f1 + c1 - f;
+            };
             if (Multi) {
-                // batch b of every phantom, laid end to end
+                // the group's histories of every phantom, laid end to end
                 hprefix[0] = 0;
                 for (int k = 0; k < nprob; ++k) {
                     long long f, c;
-                    batch_range(pdone[k], phist[k], nbatch, b, f, c);
+                    group_range(pdone[k], phist[k], f, c);
                     hfirst[k] = f;
                     hprefix[k + 1] = hprefix[k] + c;
                 }
@@ -2578,7 +2682,11 @@ struct Engine : EngineBase {
                 b0 = 0;
                 bn = hprefix[nprob];
             } else {
-                batch_range(first, n, nbatch, b, b0, bn);
+                group_range(first, n, b0, bn);
+            }
+            if (group > 1) {
+                P.slot_last = nb - 1;
+                if (!Multi) P.slot_first = (unsigned)b0;
             }
             for (long long c0 = b0, cn = 0; c0 < b0 + bn; c0 += cn) {
                 cn = std::min(chunk, b0 + bn - c0);   // the autotuner may change `chunk` below
@@ -2650,10 +2758,12 @@ struct Engine : EngineBase {
                         }
                     }
                 }
-                if (tune && cn == chunk) {
+                // (a group of batches just short of a chunk counts as one, its
+                // fullest queue scaled to the chunk)
+                if (tune && (cn == chunk || (group > 1 && cn > chunk / 2 && cn == bn))) {
                     double dt = std::chrono::duration<double>(std::chrono::steady_clock::now() - t_chunk).count();
                     double rate = cn / std::max(dt, 1e-9);
-                    unsigned peak = h[8];
+                    const double peak = (double)h[8] * ((double)chunk / (double)cn);
                     if (peak > 2 * (capacity / 3)) {
                         tuned_chunk = chunk = std::max<long long>(1024, chunk / 2);
                         tune_done = true;
@@ -2672,7 +2782,7 @@ struct Engine : EngineBase {
             if (mode) { CK(cudaStreamSynchronize(ws)); continue; }
             CK(cudaEventRecord(ev[6], ws));
             k_batch<<<std::max(1, std::min(4 * sm_count, (int)((nvox + 255) / 256))), 256, 0, ws>>>(
-                (double *)d_dose.p, (double *)d_sum.p, (double *)d_sum2.p, nvox);
+                (double *)d_dose.p, (double *)d_sum.p, (double *)d_sum2.p, nvox, nb);
             CK(cudaGetLastError());
             CK(cudaEventRecord(ev[7], ws));
             CK(cudaStreamSynchronize(ws));
@@ -2745,7 +2855,7 @@ struct Engine : EngineBase {
     int nprob = 0;
     std::vector<long long> phist;   // histories per phantom per run
     std::vector<long long> pdone;   // histories already transported per phantom
-    DevMem d_probs, d_pseeds, d_psrc, d_pvoff, d_pprefix, d_pfirst;
+    DevMem d_probs, d_pseeds, d_psrc, d_pvoff, d_pprefix, d_pfirst, d_pslot;
 
     int problems(int n, const PhantomDesc *pd, const Source *src, std::string &err) override {
         std::vector<Real> x, y, z;
@@ -2806,11 +2916,14 @@ struct Engine : EngineBase {
         CK(up(d_pvoff, voff.data(), (n + 1) * sizeof(int)));
         CK(d_pprefix.alloc((n + 1) * sizeof(long long)));
         CK(d_pfirst.alloc((n + 1) * sizeof(long long)));
+        CK(d_pslot.alloc(n * sizeof(uint2)));
+        CK(cudaMemset(d_pslot.p, 0, n * sizeof(uint2)));
         G = gs[0];
         nvox = tot;
         nprob = n;
         homogeneous = false;
         pdone.assign(n, 0);
+        dose_slots = 1;
         CK(d_dose.alloc(nvox * sizeof(double)));
         CK(d_sum.alloc(nvox * sizeof(double)));
         CK(d_sum2.alloc(nvox * sizeof(double)));

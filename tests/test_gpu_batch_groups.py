@@ -1,0 +1,83 @@
+"""Batches transported together (one tally slot each) against batches run one at
+a time: sum and sum of squares over batches.  A slot's deposits are added in
+another order (FP64 atomics), so the two agree to the chunking tolerance of the
+parity tests: about 1e3 additions of FP64 values per voxel, 1e3 * 2^-53 < 1e-12.
+FP32 runs may also merge the deposits of two particles of one history in FP32
+(6e-8 of one deposit), hence their 2e-5 bound, the scheduling tolerance there.
+"""
+import numpy as np
+import pytest
+
+import egsnrc_gb300 as eg
+from egsnrc_gb300 import workloads as W
+
+pytestmark = pytest.mark.gpu
+TOL = {64: 1e-12, 32: 2e-5}
+
+
+def ranges(n, nb):
+    per = n // nb
+    return [(b * per, per if b < nb - 1 else n - b * per) for b in range(nb)]
+
+
+def one_by_one(e, n, nb, seed):
+    s = s2 = 0
+    for first, cnt in ranges(n, nb):
+        e.reset()
+        e.run(cnt, nbatch=1, seed=seed, first=first)
+        d = e.tallies()[0]
+        s, s2 = s + d, s2 + d * d
+    return s, s2
+
+
+# chunk 0: all batches in one group; 300: groups of two whose wavefronts are
+# cut inside a batch; 40: smaller than a batch, so each batch runs alone
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("n,nb,cfg", [(1003, 7, {}), (1003, 7, {"chunk": 300}), (1003, 7, {"chunk": 40}),
+                                      (20, 20, {}), (1003, 7, {"use_graph": 1}), (1003, 7, {"use_graph": 2}),
+                                      (1003, 7, {"use_graph": 1, "chunk": 300}), (501, 1, {})])
+def test_grouped_batches_equal_single_batches(n, nb, cfg, precision):
+    wl = W.slab64(16)
+    def engine(**kw):
+        e = eg.DoseEngine(wl["media"], ecut=wl["ecut"], pcut=wl["pcut"], precision=precision, **kw)
+        e.set_geometry(wl["geometry"])
+        e.set_source(wl["source"])
+        return e
+    want = one_by_one(engine(), n, nb, 5)
+    e = engine(**cfg)
+    for _ in range(2):            # a second run finds every slot cleared
+        e.reset()
+        e.run(n, nbatch=nb, seed=5)
+        got = e.tallies()[:2]
+        for g, w in zip(got, want):
+            assert w.sum() > 0
+            assert np.allclose(g, w, rtol=TOL[precision], atol=TOL[precision] * w.max())
+    # a smaller geometry and fewer batches on the same handle
+    e.set_geometry(W.slab64(8)["geometry"])
+    e.run(60, nbatch=3, seed=6)
+    f = engine()
+    f.set_geometry(W.slab64(8)["geometry"])
+    for g, w in zip(e.tallies()[:2], one_by_one(f, 60, 3, 6)):
+        assert np.allclose(g, w, rtol=TOL[precision], atol=TOL[precision] * w.max())
+
+
+@pytest.mark.parametrize("cfg", [{}, {"chunk": 200}, {"use_graph": 2}])
+def test_grouped_batches_of_several_phantoms(cfg):
+    nb = 3
+    def phantoms(counts):
+        return [dict(W.batch_problem(k, edge=(8 + 3 * k, 8 + 3 * k)), histories=c) for k, c in enumerate(counts)]
+    counts = [100, 3, 331, 0, 57]
+    e = eg.DoseEngine(W.BATCH_MEDIA, ecut=0.7, pcut=0.01, precision=64, **cfg)
+    e.set_phantoms(phantoms(counts))
+    e.run_phantoms(nbatch=nb)
+    for k, c in enumerate(counts):
+        s, s2 = e.phantom_tallies(k)
+        if not c:
+            assert not s.any()
+            continue
+        ph = phantoms(counts)[k]
+        f = eg.DoseEngine(W.BATCH_MEDIA, ecut=0.7, pcut=0.01, precision=64)
+        f.set_geometry(ph["geometry"])
+        f.set_source(ph["source"])
+        for g, w in zip((s, s2), one_by_one(f, c, nb, ph["seed"])):
+            assert np.allclose(g, w, rtol=TOL[64], atol=TOL[64] * max(w.max(), 1e-30))
