@@ -494,11 +494,12 @@ __device__ inline void mscat(const Tables<Real> &T, Rng &r, Real lambda, Real ch
     cost = 1; sint = 0;
 }
 
-// msdist_pII, spin effects off (src/egsnrc.mortran:4050-4294)
+// msdist_pII, spin effects off (src/egsnrc.mortran:4050-4294); `lanes`: the
+// warp's lanes that take it together
 template <class Real>
 __device__ inline void msdist_pII(const Tables<Real> &T, const MedScalars<Real> &M, Particle<Real> &p, Real e0,
                                   Real eloss, Real tustep, Real rhof, Real &us, Real &vs, Real &ws, Real &xf,
-                                  Real &yf, Real &zf, int &err) {
+                                  Real &yf, Real &zf, int &err, unsigned lanes) {
     const Real rm = (Real)RM;
     Real blccc = M.blcc, xcccc = M.xcc;
     Real e = e0 - (Real)0.5 * eloss, tau = e / rm, tau2 = tau * tau, epsilon = eloss / e0, epsilonp = eloss / e;
@@ -524,6 +525,7 @@ __device__ inline void msdist_pII(const Tables<Real> &T, const MedScalars<Real> 
     for (int half = 0; half < 2; ++half) {
         Real wh, sh;
         mscat(T, p.rng, lambda, chia2, xi, st, wh, sh, err);
+        __syncwarp(lanes);
         Azim<Real> ah = azimuth<Real>(p.rng, err);
         if (half == 0) { w1 = wh; sint1 = sh; a1 = ah; } else { w2 = wh; sint2 = sh; a2 = ah; }
     }

@@ -1070,8 +1070,19 @@ __device__ __noinline__ Real wide_eloss(const Tables<Real> &T, const MedScalars<
 // carry none of this code.
 // SPL: the precision split of the FP32 kernel (egsgpu_config.fp64_near_faces),
 // its own instantiation so that the default FP32 step carries none of it.
+//
+// The step is bound by the latency of its long dependent chains, not by issue
+// (53% of cycles) or memory.  The lanes that step carry their mask (`go`) and
+// meet again after the start of a new step sequence, before the face distances
+// and after the deflection: left alone, the compiler threads the new sequences
+// past the join, and the warp ran the whole step 1.2-1.4 times per iteration in
+// two thin groups.  FP32: five CTAs per SM, the most at which nothing spills
+// (94-96 registers; six were 80 with spills).  Both together, one GB300:
+// slab64 1e8 histories 526 -> 500 ms, water128e 2e5 163 -> 156 ms, perturbed64
+// 46.0 -> 40.8 ms.  HOWFARLESS and the precision split keep six, and HOWFARLESS
+// joins only before the hinge: measured no faster otherwise.
 template <class Real, bool Multi, bool Adj = false, bool HFL = false, bool PI = false, bool SPL = false>
-__global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? 6 : 1) k_electron(Params<Real> P) {
+__global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL || SPL ? 6 : 5) : 1) k_electron(Params<Real> P) {
     const Tables<Real> &T = P.T;
     const Geom<Real> &G = P.G;
     const unsigned lane = threadIdx.x & 31u;
@@ -1409,15 +1420,18 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? 6 : 1) 
                 continue;
             }
         }
-        if (!alive || s.state == 3) continue;
+        bool step = alive && s.state != 3;
+        if (step && ++s.nsteps > STEP_CAP) { err = 1; alive = step = false; }
+        unsigned go = __ballot_sync(0xffffffffu, step);   // the lanes taking a step
+        if (!step) continue;
 
         const int qel = (1 + p.iq) / 2;
         bool ecut_discard = false;
-        if (++s.nsteps > STEP_CAP) { err = 1; alive = false; continue; }
         if (s.state == 0) {   // :NEWELECTRON:
             if (p.E <= T.ecut) ecut_discard = true;
             else s.state = 1;
         }
+        go = __ballot_sync(go, !ecut_discard);
         if (!ecut_discard) {
             if (s.state == 1) {   // :TSTEP:
                 const MedScalars<Real> &M = cmed<Real>(s.medium);
@@ -1432,6 +1446,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? 6 : 1) 
                 else s.sig0 = qel ? M.psig_e : M.esig_e;
                 s.state = 2;
             }
+            if (!HFL) __syncwarp(go);
             // :USTEP: one condensed-history step
             const MedScalars<Real> &M = cmed<Real>(s.medium);
             Real rhof = s.rhor, sig = s.sig0;
@@ -1463,6 +1478,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? 6 : 1) 
                 }
                 tstep = s.total_tstep / (Real)rhof;
             }
+            if (!HFL) __syncwarp(go);
             ERow<Real> er{erow(T, M, s.lelke), qel};
             const Real *row = er.r;
             Real dedx0 = er.dedx(s.elke), dedx = rhof * dedx0;
@@ -1528,12 +1544,13 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? 6 : 1) 
                     if (tuss < tustep) { tustep = tuss; dosingle = true; }
                 } else {
                     err = 1;
-                    alive = false;
-                    continue;
+                    alive = step = false;
                 }
                 ustep = tustep;
                 callhowfar = !(ustep < tperp);
             }
+            go = __ballot_sync(go, step);
+            if (!step) continue;
             const Real ustep0 = ustep;
             int irold = p.ir, irnew = p.ir, axis = -1;
             if (callhowfar) {
@@ -1549,20 +1566,25 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? 6 : 1) 
             }
             if (ustep <= 0) ustep = 0;
             if (ustep == 0) {
+                step = false;
                 if (irnew != irold) {
                     p.ir = irnew;
                     if (irnew < 0) {
                         esc_tot += (double)((p.iq < 0 ? p.E - rm : p.E + rm) * p.wt);
                         if (Adj) elist_flush(P, el);
                         alive = false;
-                        continue;
+                    } else {
+                        s.medium = G.med[irnew];
+                        s.rhor = G.rhor[irnew];
                     }
-                    s.medium = G.med[irnew];
-                    s.rhor = G.rhor[irnew];
                 }
-                if (p.E <= T.ecut) ecut_discard = true;
-                else { s.state = 1; continue; }
+                if (alive) {
+                    if (p.E <= T.ecut) ecut_discard = true;
+                    else s.state = 1;
+                }
             }
+            go = __ballot_sync(go, step);
+            if (!step && !ecut_discard) continue;
             if (!ecut_discard) {
                 Real vstep = ustep, tvstep = callhowfar ? vstep : tustep;
                 if (PI && callhowfar) {   // $SET-TVSTEP (src/egsnrc.macros:1350-1392)
@@ -1570,8 +1592,12 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? 6 : 1) 
                         calculate_xi(s.eke - (Real)0.5 * tustep * vstep / ustep0 * dedx, vstep);
                         if (ms_xi < (Real)0.1) tvstep = vstep * (1 + ms_xi * ((Real)0.5 + ms_xi * (Real)0.333333));
                         else if (ms_xi < (Real)0.999999) tvstep = -vstep * dlog(1 - ms_xi) / ms_xi;
-                        else { err = 1; alive = false; continue; }
+                        else { err = 1; alive = step = false; }
                     } else tvstep = tustep;
+                }
+                if (PI) {
+                    go = __ballot_sync(go, step);
+                    if (!step) continue;
                 }
                 if (!PI && callhowfar && tvstep != tustep) dosingle = false;
                 if (wide) {   // a step limited by the range ends it exactly, as in FP64
@@ -1580,7 +1606,8 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? 6 : 1) 
                 } else {
                     de = eloss_g<Real>(T, M, qel, (Real)tvstep, (Real)s.eke, (Real)s.elke, s.lelke, range, (Real)rhof);
                 }
-                if (callmsdist) msdist_pII(T, M, p, s.eke, (Real)de, tustep, rhof, uf, vf, wf, xf, yf, zf, err);
+                const unsigned ms = __ballot_sync(go, callmsdist);
+                if (callmsdist) msdist_pII(T, M, p, s.eke, (Real)de, tustep, rhof, uf, vf, wf, xf, yf, zf, err, ms);
                 Real edep = (Real)de, ekef = s.eke - edep;
                 if (!callmsdist) {
                     xf = p.x + p.u * vstep; yf = p.y + p.v * vstep; zf = p.z + p.w * vstep;
@@ -1603,6 +1630,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? 6 : 1) 
                         rotate(p.u, p.v, p.w, sinthe, costhe, az, uf, vf, wf);
                     } else { uf = p.u; vf = p.v; wf = p.w; }
                 }
+                if (!HFL) __syncwarp(go);
                 if (HFL) {
                     const Real xi0[3] = {p.x, p.y, p.z}, ui0[3] = {p.u, p.v, p.w};
                     p.x = xf; p.y = yf; p.z = zf; p.u = uf; p.v = vf; p.w = wf;
