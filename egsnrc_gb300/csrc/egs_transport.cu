@@ -115,7 +115,7 @@ struct Params {
     unsigned *peak;                       // largest queue length seen (autotuner input)
     uint32_t seed;
     int requeue_lanes;                    // park survivors of warps this sparse (0 = never)
-    int inter_batch;                      // electron lanes due to interact before the warp samples them
+    int inter_batch;                      // electron lanes due to interact before a full warp samples them
     int inter_batch_p;                    // the same for photon lanes
 };
 
@@ -271,6 +271,20 @@ __device__ inline void q_load(const Queue<Real> &q, unsigned i, uint32_t seed, P
     p.E = q.E[i]; p.wt = q.wt[i]; p.ir = q.ir[i];
     p.iq = q.iq ? (int)q.iq[i] : 0;
     p.rng.init(seed, q.hist[i], q.sid[i], q.n[i]);
+}
+// A launch whose queue holds no more particles than the grid has lanes gives
+// every warp the same number k of them (the lowest k lanes) and fetches no
+// more.  Filling whole warps instead leaves most warps of the grid empty and
+// makes each track wait, step by step, for the divergent paths of 31 others;
+// the longest track is what such a launch takes (512 slab64 histories: 2.85 ->
+// 1.71 ms, 1e4 water30 histories: 6.6 -> 4.6 ms).  Returns the warp's first
+// record.  The fetch in front of the loop is a copy of its own: a branch at the
+// fetch inside the loop cost dense launches 3%.  Not with requeue_lanes, which
+// would park such thin warps again before they took a step.
+__device__ inline unsigned sparse_share(unsigned nq, unsigned &k) {
+    const unsigned per_cta = blockDim.x >> 5, nw = gridDim.x * per_cta;
+    k = (nq + nw - 1) / nw;
+    return (blockIdx.x * per_cta + (threadIdx.x >> 5)) * k;
 }
 // The phantom holding global voxel `ir` (largest k with pvoff[k] <= ir).
 template <class Real>
@@ -708,8 +722,6 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 ? 8 : 1) k_photon
     const unsigned lane = threadIdx.x & 31u;
     const unsigned nq = *P.pin.count < P.pin.capacity ? *P.pin.count : P.pin.capacity;
     if (threadIdx.x == 0 && blockIdx.x == 0) atomicMax(P.peak, *P.pin.count);
-    __shared__ unsigned s_dummy;
-    (void)s_dummy;
     Particle<Real> p;
     PhotonState<Real> s;
     Acc<Real, Multi> acc{-1, 0u, (Real)0, 0u};
@@ -722,6 +734,35 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 ? 8 : 1) k_photon
     int err = 0;
     const Real rm = (Real)RM;
     const bool requeue = P.requeue_lanes > 0 && nq >= REQUEUE_MIN;
+    auto take = [&](unsigned idx) {   // queue record idx becomes this lane's particle
+        load_particle<Real, Multi>(P, P.pin, idx, p, acc);
+        if (Adj) Gh = hist_weight(P, p);
+        alive = true;
+        s.state = 0;
+        s.nsteps = 0;
+        if (P.pin.st[idx] == 3) {   // resume a photon due to interact
+            const MedScalars<Real> &M = cmed<Real>(G.med[p.ir]);
+            s.state = 3;
+            s.medium = G.med[p.ir];
+            s.rhor = G.rhor[p.ir];
+            s.gle = dlog(p.E);
+            s.lgle = min(max((int)(M.ge1 * s.gle + M.ge0), 1), MXGE);
+            const Real *g = T.gtab + ((size_t)M.gtab_off + s.lgle - 1) * 8;
+            s.cohfac = g[7] * s.gle + g[6];
+        } else if (P.pin.st[idx]) {   // resume a parked photon
+            s.state = 1;
+            s.medium = G.med[p.ir];
+            s.rhor = G.rhor[p.ir];
+            s.gle = dlog(p.E);
+            s.dpmfp = P.pin.aux0[idx];
+        }
+    };
+    if (!requeue && nq <= gridDim.x * blockDim.x) {
+        unsigned k;
+        const unsigned idx = sparse_share(nq, k) + lane;
+        if (lane < k && idx < nq) take(idx);
+        exhausted = true;
+    }
     while (true) {
         if (exhausted && requeue) {
             unsigned busy = __ballot_sync(0xffffffffu, alive);
@@ -745,29 +786,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 ? 8 : 1) k_photon
             if (base >= nq) exhausted = true;
             if (!alive) {
                 unsigned idx = base + __popc(need & ((1u << lane) - 1u));
-                if (idx < nq) {
-                    load_particle<Real, Multi>(P, P.pin, idx, p, acc);
-                    if (Adj) Gh = hist_weight(P, p);
-                    alive = true;
-                    s.state = 0;
-                    s.nsteps = 0;
-                    if (P.pin.st[idx] == 3) {   // resume a photon due to interact
-                        const MedScalars<Real> &M = cmed<Real>(G.med[p.ir]);
-                        s.state = 3;
-                        s.medium = G.med[p.ir];
-                        s.rhor = G.rhor[p.ir];
-                        s.gle = dlog(p.E);
-                        s.lgle = min(max((int)(M.ge1 * s.gle + M.ge0), 1), MXGE);
-                        const Real *g = T.gtab + ((size_t)M.gtab_off + s.lgle - 1) * 8;
-                        s.cohfac = g[7] * s.gle + g[6];
-                    } else if (P.pin.st[idx]) {   // resume a parked photon
-                        s.state = 1;
-                        s.medium = G.med[p.ir];
-                        s.rhor = G.rhor[p.ir];
-                        s.gle = dlog(p.E);
-                        s.dpmfp = P.pin.aux0[idx];
-                    }
-                }
+                if (idx < nq) take(idx);
             }
         }
         unsigned live = __ballot_sync(0xffffffffu, alive);
@@ -782,7 +801,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 ? 8 : 1) k_photon
             bool batch = false;
             if (pend) {
                 ++inter_wait;
-                batch = __popc(pend) >= min(P.inter_batch_p, __popc(live)) || inter_wait > INTER_MAXWAIT;
+                batch = 32 * __popc(pend) >= P.inter_batch_p * __popc(live) || inter_wait > INTER_MAXWAIT;
             }
             if (batch) {
                 inter_wait = 0;
@@ -1112,6 +1131,40 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL ||
     int err = 0;
     const Real rm = (Real)RM;
     const bool requeue = P.requeue_lanes > 0 && nq >= REQUEUE_MIN;
+    auto take = [&](unsigned idx) {   // queue record idx becomes this lane's particle
+        load_particle<Real, Multi>(P, P.ein, idx, p, acc);
+        if (Adj) el.n = 0;
+        alive = true;
+        s.state = 0;
+        s.nsteps = 0;
+        s.medium = G.med[p.ir];
+        s.rhor = G.rhor[p.ir];
+        uint8_t st = P.ein.st[idx];
+        if (st == 1) s.state = 1;
+        else if (st == 8) {   // resume a particle due to interact
+            const MedScalars<Real> &M = cmed<Real>(s.medium);
+            s.state = 3;
+            s.eke = p.E - (Real)RM;
+            s.elke = dlog(s.eke);
+            s.lelke = min(max((int)(M.eke1 * s.elke + M.eke0), 1), M.meke);
+        }
+        else if (st & 2) {   // resume a parked condensed-history sequence
+            const MedScalars<Real> &M = cmed<Real>(s.medium);
+            s.state = 2;
+            s.compute_tstep = (st & 4) ? 1 : 0;
+            s.demfp = P.ein.aux0[idx]; s.total_de = P.ein.aux1[idx];
+            s.total_tstep = P.ein.aux2[idx]; s.sig0 = P.ein.aux3[idx];
+            s.eke = p.E - (Real)RM;
+            s.elke = dlog(s.eke);
+            s.lelke = min(max((int)(M.eke1 * s.elke + M.eke0), 1), M.meke);
+        }
+    };
+    if (!requeue && nq <= gridDim.x * blockDim.x) {
+        unsigned k;
+        const unsigned idx = sparse_share(nq, k) + lane;
+        if (lane < k && idx < nq) take(idx);
+        exhausted = true;
+    }
     while (true) {
         if (!alive && sp > 0) {   // resume a suspended particle
             p = lstack[--sp];
@@ -1152,34 +1205,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL ||
                 edep_tot += (double)edep_part;
                 edep_part = 0;
                 unsigned idx = base + __popc(need & ((1u << lane) - 1u));
-                if (idx < nq) {
-                    load_particle<Real, Multi>(P, P.ein, idx, p, acc);
-                    if (Adj) el.n = 0;
-                    alive = true;
-                    s.state = 0;
-                    s.nsteps = 0;
-                    s.medium = G.med[p.ir];
-                    s.rhor = G.rhor[p.ir];
-                    uint8_t st = P.ein.st[idx];
-                    if (st == 1) s.state = 1;
-                    else if (st == 8) {   // resume a particle due to interact
-                        const MedScalars<Real> &M = cmed<Real>(s.medium);
-                        s.state = 3;
-                        s.eke = p.E - (Real)RM;
-                        s.elke = dlog(s.eke);
-                        s.lelke = min(max((int)(M.eke1 * s.elke + M.eke0), 1), M.meke);
-                    }
-                    else if (st & 2) {   // resume a parked condensed-history sequence
-                        const MedScalars<Real> &M = cmed<Real>(s.medium);
-                        s.state = 2;
-                        s.compute_tstep = (st & 4) ? 1 : 0;
-                        s.demfp = P.ein.aux0[idx]; s.total_de = P.ein.aux1[idx];
-                        s.total_tstep = P.ein.aux2[idx]; s.sig0 = P.ein.aux3[idx];
-                        s.eke = p.E - (Real)RM;
-                        s.elke = dlog(s.eke);
-                        s.lelke = min(max((int)(M.eke1 * s.elke + M.eke0), 1), M.meke);
-                    }
-                }
+                if (idx < nq) take(idx);
             }
         }
         unsigned live = __ballot_sync(0xffffffffu, alive);
@@ -1190,13 +1216,16 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL ||
         // live lanes together (Rng::ahead)
         if (alive) p.rng.ahead(RNG_AHEAD);
         // Discrete interactions are sampled for several lanes at once (see the
-        // photon kernel).
+        // photon kernel): inter_batch of 32 live lanes, and the same share of
+        // fewer, so that the few lanes left in a launch's tail do not wait for
+        // one another (FP64 slab64 2e5 histories 92.9 -> 89.1 ms, slab64 2e6
+        // 21.6 -> 20.8 ms).
         {
             unsigned pend = __ballot_sync(0xffffffffu, alive && s.state == 3);
             bool batch = false;
             if (pend) {
                 ++inter_wait;
-                batch = __popc(pend) >= min(P.inter_batch, __popc(live)) || inter_wait > INTER_MAXWAIT;
+                batch = 32 * __popc(pend) >= P.inter_batch * __popc(live) || inter_wait > INTER_MAXWAIT;
             }
             if (batch) {
                 inter_wait = 0;

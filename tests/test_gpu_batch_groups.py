@@ -81,3 +81,34 @@ def test_grouped_batches_of_several_phantoms(cfg):
         f.set_source(ph["source"])
         for g, w in zip((s, s2), one_by_one(f, c, nb, ph["seed"])):
             assert np.allclose(g, w, rtol=TOL[64], atol=TOL[64] * max(w.max(), 1e-30))
+
+
+# the sparse launch's edges: fewer particles than warps, one or two per warp, a
+# few more than the grid has lanes (about 1e5), and requeue on a sparse launch
+@pytest.mark.parametrize("n,requeue", [(1, 0), (33, 0), (5000, 0), (120000, 0), (60000, 24)])
+def test_sparse_launches_take_every_particle_once(n, requeue):
+    wl = W.water30(10)
+    t = []
+    for cfg in ({}, {"chunk": 1009, "block_size": 32, "ctas_per_sm": 1, "requeue_lanes": requeue}):
+        e = eg.DoseEngine(wl["media"], ecut=wl["ecut"], pcut=wl["pcut"], precision=32, **cfg)
+        e.set_geometry(wl["geometry"])
+        e.set_source(wl["source"])
+        e.run(n, nbatch=1, seed=9)
+        t.append((e.tallies()[0], e.totals()))
+        e.close()
+    assert t[0][1]["steps"] == t[1][1]["steps"] > 0
+    assert t[0][1]["deposited"] + t[0][1]["escaped"] == pytest.approx(2.0 * n, rel=1e-6)
+    assert np.allclose(t[0][0], t[1][0], rtol=TOL[32], atol=TOL[32] * t[0][0].max())
+
+
+def test_requeue_on_a_sparse_launch_makes_progress():
+    wl = W.water30(10)
+    t = []
+    for requeue in (0, 24):
+        e = eg.DoseEngine(wl["media"], ecut=wl["ecut"], pcut=wl["pcut"], precision=32, requeue_lanes=requeue)
+        e.set_geometry(wl["geometry"])
+        e.set_source(wl["source"])
+        e.run(60000, nbatch=1, seed=9)
+        t.append(e.totals()["steps"])
+        e.close()
+    assert t[0] == t[1] > 0
