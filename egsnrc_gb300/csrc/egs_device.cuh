@@ -161,8 +161,8 @@ static __host__ __device__ __noinline__ uint4 philox_block(uint32_t b, uint32_t 
                                                            uint32_t k1);
 
 // The generator keeps a window of the stream's next four Philox blocks
-// (block b in slot b & 3; `next` is one past the highest block held).  A
-// draw refills only when its block is missing.  The transport loops call
+// (number i in word i & 15; `lim` is one past the highest number held).  A
+// draw computes only a block that is missing.  The transport loops call
 // ahead(k) where the warp is converged, so that the blocks the lanes will
 // need for the coming step are computed there, by all lanes together, instead
 // of at whichever draw site a lane's counter happens to cross into a new block
@@ -171,13 +171,97 @@ static __host__ __device__ __noinline__ uint4 philox_block(uint32_t b, uint32_t 
 // The numbers are the same either way: the window only decides when a block
 // is computed.  A copy holds the stream position but not the window, so
 // particle copies stay small and a copy never reads blocks it did not compute.
+//
+// The window belongs to the thread: on the device it is a column of a shared
+// array (word w of thread t at [w][t], free of bank conflicts; 8 KB per CTA),
+// which leaves position, key and limit in registers and makes a draw one
+// shared-memory load, inlined.  With the window in local memory (RngLocal) the
+// whole particle lives there too, around every out-of-line draw.  Local -> shared
+// window, one GB300: water128e 2e5 histories 154 -> 136 ms, perturbed64 777777
+// 39.9 -> 36.2 ms, slab64 1e8 500 -> 494 ms.  (At 80 registers instead of 96 it
+// loses 3-10%: the particle spills.)
+// Drawing from a second Rng of the thread overwrites the first one's window: the
+// first must drop() its window before it draws again.
+constexpr int RNG_THREADS = 128;   // most threads of a CTA whose threads draw
+#ifdef __CUDA_ARCH__
+__device__ inline uint32_t *rng_window() {
+    __shared__ uint32_t w[16 * RNG_THREADS];
+    return w + threadIdx.x;
+}
+#endif
 struct Rng {
+    uint32_t seed, hist, n, lim;
+    uint64_t sid;
+#ifdef __CUDA_ARCH__
+    __device__ inline uint32_t &word(uint32_t i) { return rng_window()[i * RNG_THREADS]; }
+#else
+    uint32_t c[16];
+    uint32_t &word(uint32_t i) { return c[i]; }
+#endif
+    Rng() = default;
+    __host__ __device__ Rng(const Rng &o) : seed(o.seed), hist(o.hist), n(o.n), lim(0), sid(o.sid) {}
+    __host__ __device__ Rng &operator=(const Rng &o) {
+        seed = o.seed; hist = o.hist; n = o.n; sid = o.sid; lim = 0;
+        return *this;
+    }
+    __host__ __device__ void init(uint32_t s, uint32_t h, uint64_t id, uint32_t n0) {
+        seed = s; hist = h; sid = id; n = n0; lim = 0;
+    }
+    __host__ __device__ inline void drop() { lim = 0; }
+    __host__ __device__ inline void put(uint32_t b, uint32_t o0, uint32_t o1, uint32_t o2, uint32_t o3) {
+        const uint32_t w = (b & 3u) << 2;
+        word(w) = o0; word(w + 1) = o1; word(w + 2) = o2; word(w + 3) = o3;
+    }
+    __host__ __device__ inline void fill(uint32_t b) {
+        const uint4 o = philox_block(b, (uint32_t)sid, (uint32_t)(sid >> 32), seed, hist);
+        put(b, o.x, o.y, o.z, o.w);
+        lim = (b << 2) + 4;
+    }
+    // make the blocks holding the next k numbers (1 <= k <= 13) present.  The ten
+    // rounds are inlined here (one copy per transport loop): a call to the
+    // shared out-of-line block from this site measured 10-20% slower.
+    __host__ __device__ inline void ahead(uint32_t k) {
+        const uint32_t b0 = n >> 2, b1 = (n + k - 1) >> 2;
+        uint32_t b = (lim >> 2) > b0 ? lim >> 2 : b0;
+        for (; b <= b1; ++b) {
+            uint32_t o[4];
+            philox10(b, (uint32_t)sid, (uint32_t)(sid >> 32), 0u, seed, hist, o);
+            put(b, o[0], o[1], o[2], o[3]);
+        }
+        if ((b << 2) > lim) lim = b << 2;
+    }
+    __host__ __device__ inline float u() { return draw(); }
+    __host__ __device__ inline float2 u2() {
+        float a = draw();
+        return make_float2(a, draw());
+    }
+    __host__ __device__ inline float draw() {
+        // present: n < lim, and n >= lim - 16 since ahead() never runs more
+        // than three blocks past the current one
+        if (n >= lim) fill(n >> 2);
+        const uint32_t x = word(n & 15u);
+        ++n;
+        // (x >> 9) + 0.5 scaled by 2^-23: exact in FP32 and FP64, in (0,1).  The
+        // fused form has the same value and cannot be fused again into the
+        // caller's expression, whose rounding must not depend on inlining.
+#ifdef __CUDA_ARCH__
+        return __fmaf_rn((float)(x >> 9), 1.0f / 8388608.0f, 1.0f / 16777216.0f);
+#else
+        return ((float)(x >> 9) + 0.5f) * (1.0f / 8388608.0f);
+#endif
+    }
+};
+// The same generator with its window in the object, so in local memory, and
+// its draws out of line: for the source kernel, and for the kernels whose own
+// state leaves no registers for the position and key (HOWFARLESS, the precision
+// split and the adjoint: with the shared window HOWFARLESS runs 8% slower).
+struct RngLocal {
     uint32_t seed, hist, n, next;
     uint64_t sid;
     alignas(16) uint32_t c[16];
-    Rng() = default;
-    __host__ __device__ Rng(const Rng &o) : seed(o.seed), hist(o.hist), n(o.n), next(0), sid(o.sid) {}
-    __host__ __device__ Rng &operator=(const Rng &o) {
+    RngLocal() = default;
+    __host__ __device__ RngLocal(const RngLocal &o) : seed(o.seed), hist(o.hist), n(o.n), next(0), sid(o.sid) {}
+    __host__ __device__ RngLocal &operator=(const RngLocal &o) {
         seed = o.seed; hist = o.hist; n = o.n; sid = o.sid; next = 0;
         return *this;
     }
@@ -187,6 +271,7 @@ struct Rng {
     __host__ __device__ inline void fill(uint32_t b) {
         reinterpret_cast<uint4 *>(c)[b & 3u] = philox_block(b, (uint32_t)sid, (uint32_t)(sid >> 32), seed, hist);
     }
+    __host__ __device__ inline void drop() { next = 0; }
     // make the blocks holding the next k numbers (1 <= k <= 13) present.  The ten
     // rounds are inlined here (one copy per transport loop): a call to the
     // shared out-of-line block from this site measured 10-20% slower.
@@ -223,10 +308,11 @@ struct Rng {
     }
 };
 // Uniform in (0,1) with 23 random bits: the same value in FP32 and FP64.
-template <class Real>
-__device__ inline Real urand(Rng &r) { return (Real)r.u(); }
+template <class Real, class R>
+__device__ inline Real urand(R &r) { return (Real)r.u(); }
 // two consecutive uniforms in one call (the same numbers as two urand calls)
-__device__ inline float2 urand2(Rng &r) { return r.u2(); }
+template <class R>
+__device__ inline float2 urand2(R &r) { return r.u2(); }
 
 // --------------------------------------------------------- math shims ----
 // FP32 transport uses the SFU-based intrinsics; FP64 uses the full-precision
@@ -242,5 +328,16 @@ __device__ inline double dcos(double x) { return cos(x); }
 template <class T> __device__ inline T dmin(T a, T b) { return a < b ? a : b; }
 template <class T> __device__ inline T dmax(T a, T b) { return a > b ? a : b; }
 template <class T> __device__ inline T dabs(T a) { return a < 0 ? -a : a; }
+// Sums of products with their rounding written out: which product of a sum the
+// compiler fuses depends on the code around it (inlining, spills, where values
+// live), and the FP32 results must not.  The FP64 build fuses nothing.
+__device__ inline float rmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ inline double rmul(double a, double b) { return a * b; }
+__device__ inline float radd(float a, float b) { return __fadd_rn(a, b); }
+__device__ inline double radd(double a, double b) { return a + b; }
+__device__ inline float rfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ inline double rfma(double a, double b, double c) { return a * b + c; }
+template <class T> __device__ inline T sum2(T a, T b, T c, T d) { return rfma(a, b, rmul(c, d)); }    // a b + c d
+template <class T> __device__ inline T dif2(T a, T b, T c, T d) { return rfma(a, b, -rmul(c, d)); }   // a b - c d
 
 }  // namespace egsgpu

@@ -2,31 +2,66 @@
 // (paths relative to HEN_HOUSE) and draws its random numbers from the
 // interacting particle's own Philox stream, in the reference's order.
 #pragma once
+#include <type_traits>
+
 #include "egs_device.cuh"
 
 namespace egsgpu {
 
-template <class Real>
+template <class Real, class R = Rng>
 struct Particle {
     Real x, y, z, u, v, w, E, wt;
     int ir, iq;
     int pb;       // phantom of a multi-phantom run (derived from ir; not stored in queues)
-    Rng rng;
+    R rng;
 };
 
 template <class Real>
 struct Azim { Real c, s; };
 
 // $SELECT-AZIMUTHAL-ANGLE (src/egsnrc.macros:2491-2509)
-// out of line: see Rng::u (egs_device.cuh)
+// One copy out of line for its ten call sites (inlined copies cost more in
+// instruction fetch than the calls); the generator goes in and out by value, in
+// registers.
 template <class Real>
-__device__ __noinline__ Azim<Real> azimuth(Rng &r, int &err) {
+struct AzimDraw {
+    Real c, s;
+    uint32_t n, lim;
+    int err;
+};
+template <class Real>
+__device__ __noinline__ AzimDraw<Real> azimuth_draw(uint32_t n, uint32_t lim, uint32_t seed, uint32_t hist, uint64_t sid) {
+    Rng r;
+    r.n = n; r.lim = lim; r.seed = seed; r.hist = hist; r.sid = sid;
+    Real xphi, xphi2, yphi, yphi2, rho2;
+    int it = 0, err = 0;
+    do {
+        float2 q = urand2(r);
+        xphi = (Real)q.x; xphi = 2 * xphi - 1; xphi2 = rmul(xphi, xphi);
+        yphi = (Real)q.y; yphi2 = rmul(yphi, yphi);
+        rho2 = xphi2 + yphi2;
+        if (++it > LOOP_CAP) { err = 1; break; }
+    } while (rho2 > 1);
+    rho2 = 1 / rho2;
+    return {(xphi2 - yphi2) * rho2, 2 * xphi * yphi * rho2, r.n, r.lim, err};
+}
+template <class Real>
+__device__ inline Azim<Real> azimuth(Rng &r, int &err) {
+    const AzimDraw<Real> a = azimuth_draw<Real>(r.n, r.lim, r.seed, r.hist, r.sid);
+    r.n = a.n;
+    r.lim = a.lim;
+    err |= a.err;
+    return {a.c, a.s};
+}
+
+template <class Real>
+__device__ __noinline__ Azim<Real> azimuth(RngLocal &r, int &err) {
     Real xphi, xphi2, yphi, yphi2, rho2;
     int it = 0;
     do {
         float2 q = urand2(r);
-        xphi = (Real)q.x; xphi = 2 * xphi - 1; xphi2 = xphi * xphi;
-        yphi = (Real)q.y; yphi2 = yphi * yphi;
+        xphi = (Real)q.x; xphi = 2 * xphi - 1; xphi2 = rmul(xphi, xphi);
+        yphi = (Real)q.y; yphi2 = rmul(yphi, yphi);
         rho2 = xphi2 + yphi2;
         if (++it > LOOP_CAP) { err = 1; break; }
     } while (rho2 > 1);
@@ -38,33 +73,35 @@ __device__ __noinline__ Azim<Real> azimuth(Rng &r, int &err) {
 template <class Real>
 __device__ inline void rotate(Real a, Real b, Real c, Real sinthe, Real costhe, Azim<Real> az, Real &u,
                               Real &v, Real &w) {
-    Real sinps2 = a * a + b * b;
+    Real sinps2 = sum2(a, a, b, b);
     if (sinps2 < (Real)1e-20) {
         u = sinthe * az.c; v = sinthe * az.s; w = c * costhe;
     } else {
         Real sinpsi = dsqrt(sinps2), us = sinthe * az.c, vs = sinthe * az.s;
         Real sindel = b / sinpsi, cosdel = a / sinpsi;
-        u = c * cosdel * us - sindel * vs + a * costhe;
-        v = c * sindel * us + cosdel * vs + b * costhe;
-        w = -sinpsi * us + c * costhe;
+        u = rfma(a, costhe, dif2(c * cosdel, us, sindel, vs));
+        v = rfma(b, costhe, sum2(c * sindel, us, cosdel, vs));
+        w = dif2(c, costhe, sinpsi, us);
     }
 }
 
 // ------------------------------------------------------------ Rayleigh ----
 // egs_rayleigh_sampling (src/egsnrc.mortran:8559-8590)
-template <class Real>
-__device__ inline void rayleigh(const Tables<Real> &T, int med, Real E, Real gle, int lgle, Rng &r,
+template <class Real, class R>
+__device__ inline void rayleigh(const Tables<Real> &T, int med, Real E, Real gle, int lgle, R &r,
                                 Real &costhe, Real &sinthe, int &err) {
     const Real hc_i = (Real)80.65506856998, twice_hc2 = (Real)0.000307444456, dwi = (Real)(NRAY - 1);
     const Real *pm = T.pmax + ((size_t)med * MXGE + (lgle - 1)) * 2;
     const Real *xg = T.ray + (size_t)med * 4 * NRAY, *fc = xg + NRAY, *ba = fc + NRAY, *ca = ba + NRAY;
     const int *ia = T.ray_i + (size_t)med * NRAY;
     Real pmax = pm[1] * gle + pm[0], xmax = hc_i * E, xv, csq, rn1;
+    constexpr bool own = std::is_same<R, Rng>::value;   // written-out rounding (RngLocal: the compiler's)
     int it = 0;
     do {
         rn1 = urand<Real>(r);
         do {
-            Real r0 = urand<Real>(r) * pmax;
+            const Real q = urand<Real>(r);
+            Real r0 = own ? rmul(q, pmax) : q * pmax;
             int ibin = 1 + (int)(r0 * dwi);
             int ib = ia[ibin - 1];
             if (ia[ibin] > ib) {
@@ -76,7 +113,7 @@ __device__ inline void rayleigh(const Tables<Real> &T, int med, Real E, Real gle
         } while (!(xv < xmax));
         xv = xv / E;
         costhe = 1 - twice_hc2 * xv * xv;
-        csq = costhe * costhe;
+        csq = own ? rmul(costhe, costhe) : costhe * costhe;
         if (it > LOOP_CAP) break;
     } while (!(2 * rn1 < 1 + csq));
     sinthe = dsqrt(dmax((Real)0, 1 - csq));
@@ -87,10 +124,10 @@ __device__ inline void rayleigh(const Tables<Real> &T, int med, Real E, Real gle
 // The photon is updated in place; the electron direction/energy returned.
 // Returns the binding energy deposited locally (relaxation products are all
 // below the transport cut-offs, which the host checks).
-template <class Real>
-__device__ inline Real compton(const Tables<Real> &T, const MedScalars<Real> &M, Particle<Real> &p,
+template <class Real, class R>
+__device__ inline Real compton(const Tables<Real> &T, const MedScalars<Real> &M, Particle<Real, R> &p,
                                Real &eu, Real &ev, Real &ew, Real &eE, int &err) {
-    Rng &r = p.rng;
+    R &r = p.rng;
     const Real rm = (Real)RM;
     Real peig = p.E, ko = peig / rm, broi = 1 + 2 * ko;
     bool first_time = true;
@@ -230,10 +267,10 @@ __device__ inline Real compton(const Tables<Real> &T, const MedScalars<Real> &M,
 // PHOTO with EADL edges (src/egsnrc.mortran:5050-5195) and the Sauter
 // photo-electron direction (src/egsnrc.macros:1916-1955). Converts p into the
 // photo-electron; returns the vacancy energy deposited locally.
-template <class Real>
-__device__ inline Real photo(const Tables<Real> &T, const MedScalars<Real> &M, Particle<Real> &p, Real gle,
+template <class Real, class R>
+__device__ inline Real photo(const Tables<Real> &T, const MedScalars<Real> &M, Particle<Real, R> &p, Real gle,
                              int &err) {
-    Rng &r = p.rng;
+    R &r = p.rng;
     const Real rm = (Real)RM;
     Real peig = p.E, e_vac = 0;
     const Real *el;
@@ -317,10 +354,10 @@ __device__ inline Real photo(const Tables<Real> &T, const MedScalars<Real> &M, P
 // ---------------------------------------------------------------- PAIR ----
 // PAIR (src/egsnrc.mortran:4518-4715) with $SET-PAIR-ANGLE iprdst = 1
 // (src/egsnrc.macros:2070-2125) and the low-energy uniform split (:2179-2185).
-template <class Real>
-__device__ inline void pair(const MedScalars<Real> &M, Particle<Real> &p, Real &E2, int &iq2, Real &u2, Real &v2,
+template <class Real, class R>
+__device__ inline void pair(const MedScalars<Real> &M, Particle<Real, R> &p, Real &E2, int &iq2, Real &u2, Real &v2,
                             Real &w2, int &err) {
-    Rng &r = p.rng;
+    R &r = p.rng;
     const Real rm = (Real)RM, rmt2 = (Real)(2 * RM);
     Real peig = p.E, eig = peig, pese1, pese2;
     int iq1;
@@ -401,8 +438,8 @@ template <class Real>
 struct MsState { bool find_index; int i, j; Real omega2; };
 
 // mscat, spin effects off (src/egsnrc.mortran:2984-3136)
-template <class Real>
-__device__ inline void mscat(const Tables<Real> &T, Rng &r, Real lambda, Real chia2, Real q1, MsState<Real> &st,
+template <class Real, class R>
+__device__ inline void mscat(const Tables<Real> &T, R &r, Real lambda, Real chia2, Real q1, MsState<Real> &st,
                              Real &cost, Real &sint, int &err) {
     if (lambda <= (Real)13.8) {
         Real sprob = urand<Real>(r), explambda = dexp(-lambda);
@@ -496,14 +533,14 @@ __device__ inline void mscat(const Tables<Real> &T, Rng &r, Real lambda, Real ch
 
 // msdist_pII, spin effects off (src/egsnrc.mortran:4050-4294); `lanes`: the
 // warp's lanes that take it together
-template <class Real>
-__device__ inline void msdist_pII(const Tables<Real> &T, const MedScalars<Real> &M, Particle<Real> &p, Real e0,
+template <class Real, class R>
+__device__ inline void msdist_pII(const Tables<Real> &T, const MedScalars<Real> &M, Particle<Real, R> &p, Real e0,
                                   Real eloss, Real tustep, Real rhof, Real &us, Real &vs, Real &ws, Real &xf,
                                   Real &yf, Real &zf, int &err, unsigned lanes) {
     const Real rm = (Real)RM;
     Real blccc = M.blcc, xcccc = M.xcc;
     Real e = e0 - (Real)0.5 * eloss, tau = e / rm, tau2 = tau * tau, epsilon = eloss / e0, epsilonp = eloss / e;
-    e = e * (1 - epsilonp * epsilonp * (6 + 10 * tau + 5 * tau2) / (24 * tau2 + 72 * tau + 48));
+    e = e * (1 - epsilonp * epsilonp * (6 + 10 * tau + 5 * tau2) / (sum2((Real)72, tau, (Real)24, tau2) + 48));
     Real p2 = e * (e + 2 * rm), beta2 = p2 / (p2 + rm * rm);
     Real chia2 = xcccc / (4 * p2 * blccc);
     Real lambda = (Real)0.5 * tustep * rhof * blccc / beta2;
@@ -530,10 +567,10 @@ __device__ inline void msdist_pII(const Tables<Real> &T, const MedScalars<Real> 
         if (half == 0) { w1 = wh; sint1 = sh; a1 = ah; } else { w2 = wh; sint2 = sh; a2 = ah; }
     }
     Real cphi1 = a1.c, sphi1 = a1.s, cphi2 = a2.c, sphi2 = a2.s;
-    Real u2 = sint2 * cphi2, v2 = sint2 * sphi2, u2p = w1 * u2 + sint1 * w2;
-    us = u2p * cphi1 - v2 * sphi1;
-    vs = u2p * sphi1 + v2 * cphi1;
-    ws = w1 * w2 - sint1 * u2;
+    Real u2 = sint2 * cphi2, v2 = sint2 * sphi2, u2p = sum2(sint1, w2, w1, u2);
+    us = dif2(u2p, cphi1, v2, sphi1);
+    vs = sum2(v2, cphi1, u2p, sphi1);
+    ws = dif2(w1, w2, sint1, u2);
     xi = 2 * xi;
     Real eta = urand<Real>(p.rng);
     eta = dsqrt(eta);
@@ -548,25 +585,25 @@ __device__ inline void msdist_pII(const Tables<Real> &T, const MedScalars<Real> 
                                                               (chilog * (1 + 2 * chia2) - 2)) - (Real)0.25 * temp * temp);
     Real b = eta * delta, c = eta * (1 - delta);
     Real w1v2 = w1 * v2;
-    Real ut = b * sint1 * cphi1 + c * (cphi1 * u2 - sphi1 * w1v2) + eta1 * us * temp1;
-    Real vt = b * sint1 * sphi1 + c * (sphi1 * u2 + cphi1 * w1v2) + eta1 * vs * temp1;
-    Real wt = eta1 * (1 + temp) + b * w1 + c * w2 + eta1 * ws * temp1;
+    Real ut = rfma(eta1 * us, temp1, sum2(b * sint1, cphi1, c, dif2(cphi1, u2, sphi1, w1v2)));
+    Real vt = rfma(eta1 * vs, temp1, sum2(b * sint1, sphi1, c, sum2(sphi1, u2, cphi1, w1v2)));
+    Real wt = rfma(eta1 * ws, temp1, rfma(c, w2, sum2(eta1, 1 + temp, b, w1)));
     Real u0 = p.u, v0 = p.v, w0 = p.w;
-    Real sint02 = u0 * u0 + v0 * v0;
+    Real sint02 = sum2(u0, u0, v0, v0);
     if (sint02 > (Real)1e-20) {
         Real sint0 = dsqrt(sint02), sint0i = 1 / sint0, cphi0 = sint0i * u0, sphi0 = sint0i * v0;
-        u2p = w0 * us + sint0 * ws;
-        ws = w0 * ws - sint0 * us;
-        us = u2p * cphi0 - vs * sphi0;
-        vs = u2p * sphi0 + vs * cphi0;
-        u2p = w0 * ut + sint0 * wt;
-        wt = w0 * wt - sint0 * ut;
-        ut = u2p * cphi0 - vt * sphi0;
-        vt = u2p * sphi0 + vt * cphi0;
+        u2p = sum2(w0, us, sint0, ws);
+        ws = dif2(w0, ws, sint0, us);
+        us = dif2(u2p, cphi0, vs, sphi0);
+        vs = sum2(u2p, sphi0, vs, cphi0);
+        u2p = sum2(w0, ut, sint0, wt);
+        wt = dif2(w0, wt, sint0, ut);
+        ut = dif2(u2p, cphi0, vt, sphi0);
+        vt = sum2(u2p, sphi0, vt, cphi0);
     } else { wt = w0 * wt; ws = w0 * ws; }
-    xf = p.x + tustep * ut;
-    yf = p.y + tustep * vt;
-    zf = p.z + tustep * wt;
+    xf = rfma(tustep, ut, p.x);
+    yf = rfma(tustep, vt, p.y);
+    zf = rfma(tustep, wt, p.z);
 }
 
 }  // namespace egsgpu

@@ -33,6 +33,7 @@
 #include <mutex>
 #include <string>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/egsgpu.h"
@@ -133,7 +134,7 @@ constexpr int INTER_MAXWAIT = 24;   // longest wait of a lane due to interact
 // deflections, two azimuths, the lateral displacement), plus one for a new
 // step length and one for the fictitious-cross-section test.
 constexpr unsigned RNG_AHEAD = 13;
-constexpr int MAX_BLOCK = 128;      // launch bound of the transport kernels (threads per CTA)
+constexpr int MAX_BLOCK = RNG_THREADS;   // launch bound of the transport kernels (threads per CTA)
 constexpr double VERY_FAR = 1e30;   // egs++ veryFar (egs++/egs_functions.h:105)
 // Distance to a voxel face (cm) within which an FP32 electron step is computed
 // in FP64 when the precision split is on: 2^-12 cm, about 250 FP32 units in
@@ -248,15 +249,15 @@ __device__ inline void elist_cross(EList<Real> &L, int axis, Real ua, Real coef)
     for (int i = 0; i < L.n; ++i) L.k[i] += f * L.c[i][axis];
 }
 // G_h of the particle's history in an adjoint replay
-template <class Real>
-__device__ inline Real hist_weight(const Params<Real> &P, const Particle<Real> &p) {
+template <class Real, class R>
+__device__ inline Real hist_weight(const Params<Real> &P, const Particle<Real, R> &p) {
     long long i = (long long)p.rng.hist - P.hist_first;
     return (i >= 0 && i < P.hist_n) ? (Real)P.hist_G[i] : (Real)0;
 }
 
 // ------------------------------------------------------------- queues ----
-template <class Real>
-__device__ inline void q_store(const Queue<Real> &q, unsigned i, const Particle<Real> &p) {
+template <class Real, class R>
+__device__ inline void q_store(const Queue<Real> &q, unsigned i, const Particle<Real, R> &p) {
     q.x[i] = p.x; q.y[i] = p.y; q.z[i] = p.z;
     q.u[i] = p.u; q.v[i] = p.v; q.w[i] = p.w;
     q.E[i] = p.E; q.wt[i] = p.wt; q.ir[i] = p.ir;
@@ -264,8 +265,8 @@ __device__ inline void q_store(const Queue<Real> &q, unsigned i, const Particle<
     q.hist[i] = p.rng.hist; q.n[i] = p.rng.n; q.sid[i] = p.rng.sid;
     q.st[i] = 0;
 }
-template <class Real>
-__device__ inline void q_load(const Queue<Real> &q, unsigned i, uint32_t seed, Particle<Real> &p) {
+template <class Real, class R>
+__device__ inline void q_load(const Queue<Real> &q, unsigned i, uint32_t seed, Particle<Real, R> &p) {
     p.x = q.x[i]; p.y = q.y[i]; p.z = q.z[i];
     p.u = q.u[i]; p.v = q.v[i]; p.w = q.w[i];
     p.E = q.E[i]; p.wt = q.wt[i]; p.ir = q.ir[i];
@@ -298,8 +299,8 @@ __device__ inline int phantom_of(const Params<Real> &P, int ir) {
 }
 // Loads queue record i; in a multi-phantom run the particle's phantom (and
 // with it its Philox seed) follows from its voxel index.
-template <class Real, bool Multi>
-__device__ inline void load_particle(const Params<Real> &P, const Queue<Real> &q, unsigned i, Particle<Real> &p,
+template <class Real, bool Multi, class R>
+__device__ inline void load_particle(const Params<Real> &P, const Queue<Real> &q, unsigned i, Particle<Real, R> &p,
                                      Acc<Real, Multi> &acc) {
     if (Multi) {
         int k = phantom_of(P, q.ir[i]);
@@ -330,9 +331,9 @@ __device__ inline unsigned q_slot(const Params<Real> &P, const Queue<Real> &q) {
     atomicExch(P.error + 0, 1);
     return ~0u;
 }
-template <class Real>
-__device__ inline void q_push(const Params<Real> &P, const Queue<Real> &q, const Particle<Real> &p,
-                              unsigned long long &npush) {
+template <class Real, class R>
+__device__ inline void q_push(const Params<Real> &P, const Queue<Real> &q, const Particle<Real, R> &p,
+                              unsigned &npush) {
     unsigned i = q_slot(P, q);
     if (i != ~0u) {
         q_store(q, i, p);
@@ -342,15 +343,15 @@ __device__ inline void q_push(const Params<Real> &P, const Queue<Real> &q, const
 
 // ANNIH_AT_REST (src/egsnrc.mortran:186-223): two back-to-back photons of
 // rest energy, the first continuing the positron's stream.
-template <class Real>
-__device__ inline void annih_at_rest(const Params<Real> &P, const Queue<Real> &qp, Particle<Real> &p,
-                                     unsigned long long &npush, int &err) {
+template <class Real, class R>
+__device__ inline void annih_at_rest(const Params<Real> &P, const Queue<Real> &qp, Particle<Real, R> &p,
+                                     unsigned &npush, int &err) {
     const Real rm = (Real)RM;
     Real costhe = urand<Real>(p.rng);
     costhe = 2 * costhe - 1;
     Real sinthe = dsqrt(dmax((Real)0, (1 - costhe) * (1 + costhe)));
     Azim<Real> az = azimuth<Real>(p.rng, err);
-    Particle<Real> g1 = p, g2 = p;
+    Particle<Real, R> g1 = p, g2 = p;
     g1.E = rm; g1.iq = 0; g1.u = sinthe * az.c; g1.v = sinthe * az.s; g1.w = costhe;
     g2.rng.init(p.rng.seed, p.rng.hist, child_sid(p.rng.sid, p.rng.n, 0), 0u);
     g2.E = rm; g2.iq = 0; g2.u = -g1.u; g2.v = -g1.v; g2.w = -g1.w;
@@ -361,9 +362,9 @@ __device__ inline void annih_at_rest(const Params<Real> &P, const Queue<Real> &q
 // Queue a new electron/positron, or -- when it is already at or below the
 // cut-off -- do its :ECUT-DISCARD: right here (deposit, and annihilation at
 // rest for a positron, on its own stream): what ELECTR would do first.
-template <class Real, bool Multi>
+template <class Real, bool Multi, class R>
 __device__ inline void push_charged(const Params<Real> &P, const Queue<Real> &qe, const Queue<Real> &qp,
-                                    Particle<Real> &q, Acc<Real, Multi> &acc, unsigned long long &npush,
+                                    Particle<Real, R> &q, Acc<Real, Multi> &acc, unsigned &npush,
                                     double &edep_tot, int &err) {
     if (q.E <= P.T.ecut) {
         Real edep = q.E - (Real)RM;
@@ -477,22 +478,22 @@ __device__ inline int howfar_from_out(const Geom<Real> &G, const double pos[3], 
 // DOSXYZnrc ihowfarless = 1 in a homogeneous phantom (dosxyznrc.mortran
 // HOWFAR :4177-4200, HOWNEAR :4351-4355): particles see only the phantom's
 // outer faces; voxels matter for scoring alone.
-template <class Real>
-__device__ inline Real hfl_dist_out(const Geom<Real> &G, const Particle<Real> &p) {
+template <class Real, class R>
+__device__ inline Real hfl_dist_out(const Geom<Real> &G, const Particle<Real, R> &p) {
     Real d = (Real)1e20;
     if (p.u > 0) d = dmin(d, (G.xb[G.nx] - p.x) / p.u); else if (p.u < 0) d = dmin(d, (G.xb[0] - p.x) / p.u);
     if (p.v > 0) d = dmin(d, (G.yb[G.ny] - p.y) / p.v); else if (p.v < 0) d = dmin(d, (G.yb[0] - p.y) / p.v);
     if (p.w > 0) d = dmin(d, (G.zb[G.nz] - p.z) / p.w); else if (p.w < 0) d = dmin(d, (G.zb[0] - p.z) / p.w);
     return d;
 }
-template <class Real>
-__device__ inline Real hfl_hownear(const Geom<Real> &G, const Particle<Real> &p) {
+template <class Real, class R>
+__device__ inline Real hfl_hownear(const Geom<Real> &G, const Particle<Real, R> &p) {
     Real t = dmin(p.x - G.xb[0], G.xb[G.nx] - p.x);
     t = dmin(t, dmin(p.y - G.yb[0], G.yb[G.ny] - p.y));
     return dmin(t, dmin(p.z - G.zb[0], G.zb[G.nz] - p.z));
 }
-template <class Real>
-__device__ inline int hfl_howfar(const Geom<Real> &G, const Particle<Real> &p, Real &t) {
+template <class Real, class R>
+__device__ inline int hfl_howfar(const Geom<Real> &G, const Particle<Real, R> &p, Real &t) {
     Real d = hfl_dist_out(G, p);
     if (d <= t) { t = (d <= G.bt) ? G.hbt : d; return -1; }
     return p.ir;
@@ -521,8 +522,8 @@ __device__ inline int hfl_locate(const Geom<Real> &G, Real x, Real y, Real z) {
 // cross in proportion to the path length in each.  p.ir holds the start.
 // Returns the voxel at the end of the segments, or -1 when they leave the
 // phantom; `lost` is then the energy past that point, not deposited.
-template <class Real, bool Multi>
-__device__ int hfl_hinge(const Params<Real> &P, Acc<Real, Multi> &acc, const Geom<Real> &G, Particle<Real> &p,
+template <class Real, bool Multi, class R>
+__device__ int hfl_hinge(const Params<Real> &P, Acc<Real, Multi> &acc, const Geom<Real> &G, Particle<Real, R> &p,
                          const Real xi0[3], const Real ui0[3], Real tv, bool ch_step, Real edep, Real &lost, int &err) {
     lost = 0;
     const int loc = p.ir;
@@ -634,7 +635,7 @@ __global__ void k_source(Params<Real> P, Source S0, long long first, long long n
         seed = P.pseeds[k];
     }
     const Source &S = Multi ? P.psrc[k] : S0;
-    Particle<Real> p;
+    Particle<Real, RngLocal> p;
     p.rng.init(seed, hist, 0ull, 0u);
     p.pb = k;
     p.wt = 1;
@@ -690,7 +691,7 @@ __global__ void k_source(Params<Real> P, Source S0, long long first, long long n
     p.x = (Real)x; p.y = (Real)y; p.z = (Real)z;
     p.u = (Real)u; p.v = (Real)v; p.w = (Real)w;
     p.ir = ir;
-    unsigned long long np = 0;
+    unsigned np = 0;
     if (p.iq == 0) q_push(P, P.pout, p, np);
     else q_push(P, P.eout, p, np);
 }
@@ -717,25 +718,26 @@ struct PhotonState {
 // would spill ~1 KB per thread at that bound and keeps its registers.
 template <class Real, bool Multi, bool Adj = false, bool HFL = false>
 __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 ? 8 : 1) k_photon(Params<Real> P) {
+    using R = typename std::conditional<Adj || HFL, RngLocal, Rng>::type;
     const Tables<Real> &T = P.T;
     const Geom<Real> &G = P.G;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned nq = *P.pin.count < P.pin.capacity ? *P.pin.count : P.pin.capacity;
     if (threadIdx.x == 0 && blockIdx.x == 0) atomicMax(P.peak, *P.pin.count);
-    Particle<Real> p;
+    Particle<Real, R> p;
     PhotonState<Real> s;
     Acc<Real, Multi> acc{-1, 0u, (Real)0, 0u};
     AccG<Real> ga{-1, (Real)0};
     Real Gh = 0;
     bool alive = false, exhausted = false;
-    unsigned long long nstep = 0, npush = 0, ninter = 0, lanes = 0, iters = 0;
+    unsigned nstep = 0, npush = 0, ninter = 0, lanes = 0, iters = 0;
     int inter_wait = 0;   // warp-uniform iterations since the first lane became due
     double edep_tot = 0, esc_tot = 0;
     int err = 0;
     const Real rm = (Real)RM;
     const bool requeue = P.requeue_lanes > 0 && nq >= REQUEUE_MIN;
     auto take = [&](unsigned idx) {   // queue record idx becomes this lane's particle
-        load_particle<Real, Multi>(P, P.pin, idx, p, acc);
+        load_particle<Real, Multi, R>(P, P.pin, idx, p, acc);
         if (Adj) Gh = hist_weight(P, p);
         alive = true;
         s.state = 0;
@@ -828,7 +830,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 ? 8 : 1) k_photon
                     Real E2, u2, v2, w2;
                     int iq2;
                     pair(M, p, E2, iq2, u2, v2, w2, err);
-                    Particle<Real> q = p;
+                    Particle<Real, R> q = p;
                     q.E = E2; q.iq = iq2; q.u = u2; q.v = v2; q.w = w2;
                     q.rng.init(p.rng.seed, p.rng.hist, child_sid(p.rng.sid, p.rng.n, 0), 0u);
                     push_charged(P, P.ein, P.pout, p, acc, npush, edep_tot, err);
@@ -838,7 +840,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 ? 8 : 1) k_photon
                 }
                 Real gbr2 = g[5] * s.gle + g[4];
                 if (r36 < gbr2) {
-                    Particle<Real> e = p;
+                    Particle<Real, R> e = p;
                     Real edep = compton(T, M, p, e.u, e.v, e.w, e.E, err);
                     e.iq = -1;
                     e.rng.init(p.rng.seed, p.rng.hist, child_sid(p.rng.sid, p.rng.n, 0), 0u);
@@ -914,19 +916,20 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 ? 8 : 1) k_photon
     acc_flush(P, acc);
     if (Adj) gflush(P, ga);
     // block-level counter reduction via warp shuffles
+    unsigned long long nstep_w = nstep, npush_w = npush, ninter_w = ninter;
     for (int o = 16; o > 0; o >>= 1) {
-        nstep += __shfl_down_sync(0xffffffffu, nstep, o);
-        npush += __shfl_down_sync(0xffffffffu, npush, o);
-        ninter += __shfl_down_sync(0xffffffffu, ninter, o);
+        nstep_w += __shfl_down_sync(0xffffffffu, nstep_w, o);
+        npush_w += __shfl_down_sync(0xffffffffu, npush_w, o);
+        ninter_w += __shfl_down_sync(0xffffffffu, ninter_w, o);
         edep_tot += __shfl_down_sync(0xffffffffu, edep_tot, o);
         esc_tot += __shfl_down_sync(0xffffffffu, esc_tot, o);
     }
     if (lane == 0) {
-        atomicAdd(P.counters + CNT_PLANES, lanes);
-        atomicAdd(P.counters + CNT_PITER, iters);
-        atomicAdd(P.counters + CNT_PSTEP, nstep);
-        atomicAdd(P.counters + CNT_PUSH, npush);
-        atomicAdd(P.counters + CNT_INTER, ninter);
+        atomicAdd(P.counters + CNT_PLANES, (unsigned long long)lanes);
+        atomicAdd(P.counters + CNT_PITER, (unsigned long long)iters);
+        atomicAdd(P.counters + CNT_PSTEP, nstep_w);
+        atomicAdd(P.counters + CNT_PUSH, npush_w);
+        atomicAdd(P.counters + CNT_INTER, ninter_w);
         atomicAdd(P.energy + 0, edep_tot);
         atomicAdd(P.energy + 1, esc_tot);
     }
@@ -977,6 +980,19 @@ __device__ inline C drange(const Tables<Real> &T, const MedScalars<Real> &M, int
     C aux = d1 * dedxmid;
     aux = aux * (1 + 2 * aux) * (fedep / (2 - fedep)) * (fedep / (2 - fedep)) / 6;
     return fedep * e1 * dedxmid * (1 + aux);
+}
+// $COMPUTE-DRANGE + add, the last product fused into the sum
+template <class C, class Real>
+__device__ inline C drange_plus(const Tables<Real> &T, const MedScalars<Real> &M, int qel, C e1, C e2, int lel, C el1,
+                           C el2, C add) {
+    const Real *r = erow(T, M, lel);
+    C fedep = 1 - e2 / e1;
+    C elktmp = (C)0.5 * (el1 + el2 + (C)0.25 * fedep * fedep * (1 + fedep * (1 + (C)0.875 * fedep)));
+    C d0 = qel ? (C)r[6] : (C)r[4], d1 = qel ? (C)r[7] : (C)r[5];
+    C dedxmid = 1 / (d1 * elktmp + d0);
+    C aux = d1 * dedxmid;
+    aux = aux * (1 + 2 * aux) * (fedep / (2 - fedep)) * (fedep / (2 - fedep)) / 6;
+    return rfma(fedep * e1 * dedxmid, 1 + aux, add);
 }
 // $COMPUTE-ELOSS (:3290-3312)
 template <class C, class Real>
@@ -1102,19 +1118,20 @@ __device__ __noinline__ Real wide_eloss(const Tables<Real> &T, const MedScalars<
 // joins only before the hinge: measured no faster otherwise.
 template <class Real, bool Multi, bool Adj = false, bool HFL = false, bool PI = false, bool SPL = false>
 __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL || SPL ? 6 : 5) : 1) k_electron(Params<Real> P) {
+    using R = typename std::conditional<Adj || HFL || SPL, RngLocal, Rng>::type;
     const Tables<Real> &T = P.T;
     const Geom<Real> &G = P.G;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned nq = *P.ein.count < P.ein.capacity ? *P.ein.count : P.ein.capacity;
     if (threadIdx.x == 0 && blockIdx.x == 0) atomicMax(P.peak, *P.ein.count);
-    Particle<Real> p;
+    Particle<Real, R> p;
     ElecState<Real> s;
     Real edep_part = 0;   // continuous-loss deposits of the current particle
     // EGSnrc's own stack discipline for the charged secondaries of Moller and
     // Bhabha events: the primary is suspended on a small per-thread LIFO (in
     // local memory) and the secondary is followed first; a full stack spills
     // to the next electron queue.
-    Particle<Real> lstack[LSTACK];
+    Particle<Real, R> lstack[LSTACK];
     int sp = 0;
     Acc<Real, Multi> acc{-1, 0u, (Real)0, 0u};
     EList<Real> el;
@@ -1124,7 +1141,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL ||
     // coefficients zero), so that its crossings also see the parent's path
     EList<Real> elstack[Adj ? LSTACK : 1];
     bool alive = false, exhausted = false;
-    unsigned long long nstep = 0, npush = 0, ninter = 0, lanes = 0, iters = 0, nwide = 0;
+    unsigned nstep = 0, npush = 0, ninter = 0, lanes = 0, iters = 0, nwide = 0;
     constexpr bool SPLIT = sizeof(Real) == 4 && !HFL && SPL;   // the FP32 kernel's FP64 steps (`wide`)
     int inter_wait = 0;   // warp-uniform iterations since the first lane became due
     double edep_tot = 0, esc_tot = 0;
@@ -1132,7 +1149,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL ||
     const Real rm = (Real)RM;
     const bool requeue = P.requeue_lanes > 0 && nq >= REQUEUE_MIN;
     auto take = [&](unsigned idx) {   // queue record idx becomes this lane's particle
-        load_particle<Real, Multi>(P, P.ein, idx, p, acc);
+        load_particle<Real, Multi, R>(P, P.ein, idx, p, acc);
         if (Adj) el.n = 0;
         alive = true;
         s.state = 0;
@@ -1269,7 +1286,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL ||
                             Real a = p.u, b = p.v, c = p.w;
                             rotate(a, b, c, sinthe, costhe, az, p.u, p.v, p.w);
                             p.E = pese1;
-                            Particle<Real> d = p;
+                            Particle<Real, R> d = p;
                             d.rng.init(p.rng.seed, p.rng.hist, child_sid(p.rng.sid, p.rng.n, 0), 0u);
                             dcosth = h1 * (pese2 - rm) / (pese2 + rm);
                             sinthe = -dsqrt(dmax((Real)0, 1 - dcosth));
@@ -1320,7 +1337,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL ||
                                 Real a = p.u, b = p.v, c = p.w;
                                 rotate(a, b, c, sinthe, costhe, az, p.u, p.v, p.w);
                                 p.E = pese1; p.iq = iq_np;
-                                Particle<Real> d = p;
+                                Particle<Real, R> d = p;
                                 d.rng.init(p.rng.seed, p.rng.hist, child_sid(p.rng.sid, p.rng.n, 0), 0u);
                                 dcosth = h1 * (pese2 - rm) / (pese2 + rm);
                                 sinthe = -dsqrt(dmax((Real)0, 1 - dcosth));
@@ -1336,7 +1353,10 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL ||
                                 ++sp;
                                 p = d;
                             }
-                                else push_charged(P, P.eout, P.pout, d, acc, npush, edep_tot, err);
+                                else {
+                                    push_charged(P, P.eout, P.pout, d, acc, npush, edep_tot, err);
+                                    p.rng.drop();   // a positron below the cut-off drew from d's stream
+                                }
                                 s.state = 0;
                                 continue;
                             }
@@ -1357,7 +1377,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL ||
                             Real costhe = dmax((Real)-1, dmin((Real)1, (esg1 - rm) * pot / esg1));
                             Real sinthe = dsqrt(1 - costhe * costhe);
                             Azim<Real> az = azimuth<Real>(p.rng, err);
-                            Particle<Real> g1 = p, g2 = p;
+                            Particle<Real, R> g1 = p, g2 = p;
                             g1.E = esg1; g1.iq = 0;
                             rotate(aa, bb, cc, sinthe, costhe, az, g1.u, g1.v, g1.w);
                             g2.rng.init(p.rng.seed, p.rng.hist, child_sid(p.rng.sid, p.rng.n, 0), 0u);
@@ -1377,7 +1397,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL ||
                     {
                         Real peie = p.E, ekin = peie - rm, brmin = M2.ap / ekin, waux = s.elke - M2.log_ap;
                         int l = (peie < 50) ? 0 : 2, l1 = l + 1;
-                        Real a = p.u, b = p.v, c = p.w, sinpsi = a * a + b * b, sindel = 0, cosdel = 0;
+                        Real a = p.u, b = p.v, c = p.w, sinpsi = sum2(a, a, b, b), sindel = 0, cosdel = 0;
                         if (sinpsi > (Real)1e-20) { sinpsi = dsqrt(sinpsi); sindel = b / sinpsi; cosdel = a / sinpsi; }
                         Real tteie = peie / rm;
                         Real beta = dsqrt((tteie - 1) * (tteie + 1)) / tteie;
@@ -1391,7 +1411,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL ||
                             r07 = (Real)q.y;
                             Real br = brmin * dexp(r06 * waux);
                             esg = ekin * br;
-                            ese = peie - esg;
+                            ese = radd(peie, -rmul(ekin, br));
                             Real delta = esg / peie / ese * M2.delcm, aux = ese / peie, phi1, phi2;
                             if (delta < 1) {
                                 phi1 = M2.dl[0][l] + delta * (M2.dl[1][l] + delta * M2.dl[2][l]);
@@ -1431,14 +1451,14 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL ||
                         Real costhe = 1 - 2 * y2tst * y2maxi;
                         Real sinthe = dsqrt(dmax((1 - costhe) * (1 + costhe), (Real)0));
                         Azim<Real> az = azimuth<Real>(p.rng, err);
-                        Particle<Real> gph = p;
+                        Particle<Real, R> gph = p;
                         gph.rng.init(p.rng.seed, p.rng.hist, child_sid(p.rng.sid, p.rng.n, 0), 0u);
                         gph.E = esg; gph.iq = 0;
                         if (sinpsi >= (Real)1e-10) {
                             Real us = sinthe * az.c, vs = sinthe * az.s;
-                            gph.u = c * cosdel * us - sindel * vs + a * costhe;
-                            gph.v = c * sindel * us + cosdel * vs + b * costhe;
-                            gph.w = c * costhe - sinpsi * us;
+                            gph.u = rfma(a, costhe, dif2(c * cosdel, us, sindel, vs));
+                            gph.v = rfma(b, costhe, sum2(c * sindel, us, cosdel, vs));
+                            gph.w = dif2(c, costhe, sinpsi, us);
                         } else { gph.u = sinthe * az.c; gph.v = sinthe * az.s; gph.w = c * costhe; }
                         q_push(P, P.pout, gph, npush);
                         p.E = ese;
@@ -1475,7 +1495,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL ||
                 else s.sig0 = qel ? M.psig_e : M.esig_e;
                 s.state = 2;
             }
-            if (!HFL) __syncwarp(go);
+            if (!HFL && !SPL) __syncwarp(go);
             // :USTEP: one condensed-history step
             const MedScalars<Real> &M = cmed<Real>(s.medium);
             Real rhof = s.rhor, sig = s.sig0;
@@ -1498,8 +1518,8 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL ||
                         else {
                             const Real *rf = rrow(T, M, lelkef + 1);
                             Real ekei = rf[0], elkei = (lelkef + 1 - (Real)M.eke0) / (Real)M.eke1;
-                            tstep = drange<Real>(T, M, qel, ekei, ekef, lelkef, elkei, elkef);
-                            tstep = tstep + r0 + rr[1 + qel] - rf[1 + qel];
+                            tstep = drange_plus<Real>(T, M, qel, ekei, ekef, lelkef, elkei, elkef, r0);
+                            tstep = tstep + rr[1 + qel] - rf[1 + qel];
                         }
                     }
                     s.total_tstep = tstep;
@@ -1507,12 +1527,12 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL ||
                 }
                 tstep = s.total_tstep / (Real)rhof;
             }
-            if (!HFL) __syncwarp(go);
+            if (!HFL && !SPL) __syncwarp(go);
             ERow<Real> er{erow(T, M, s.lelke), qel};
             const Real *row = er.r;
             Real dedx0 = er.dedx(s.elke), dedx = rhof * dedx0;
             Real tmxs = (row[15] * s.elke + row[14]) / rhof;
-            Real range = (r0 + rr[1 + qel]) / (Real)rhof;
+            Real range = radd(r0, rr[1 + qel]) / (Real)rhof;
             tmxs = dmin(tmxs, T.smaxir);
             Real tustep = (Real)dmin(tstep, dmin((Real)tmxs, range));
             const Geom<Real> &GP = geom_of<Real, Multi>(P, p.pb);
@@ -1639,7 +1659,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL ||
                 if (callmsdist) msdist_pII(T, M, p, s.eke, (Real)de, tustep, rhof, uf, vf, wf, xf, yf, zf, err, ms);
                 Real edep = (Real)de, ekef = s.eke - edep;
                 if (!callmsdist) {
-                    xf = p.x + p.u * vstep; yf = p.y + p.v * vstep; zf = p.z + p.w * vstep;
+                    xf = rfma(p.u, vstep, p.x); yf = rfma(p.v, vstep, p.y); zf = rfma(p.w, vstep, p.z);
                     if (dosingle) {   // sscat (src/egsnrc.mortran:3226-3262)
                         Real ekems = dmax(ekef, T.ecut - rm);
                         Real pp2 = ekems * (ekems + 2 * rm);
@@ -1659,7 +1679,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL ||
                         rotate(p.u, p.v, p.w, sinthe, costhe, az, uf, vf, wf);
                     } else { uf = p.u; vf = p.v; wf = p.w; }
                 }
-                if (!HFL) __syncwarp(go);
+                if (!HFL && !SPL) __syncwarp(go);
                 if (HFL) {
                     const Real xi0[3] = {p.x, p.y, p.z}, ui0[3] = {p.u, p.v, p.w};
                     p.x = xf; p.y = yf; p.z = zf; p.u = uf; p.v = vf; p.w = wf;
@@ -1730,21 +1750,22 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL ||
     }
     acc_flush(P, acc);
     edep_tot += (double)edep_part;
+    unsigned long long nstep_w = nstep, npush_w = npush, ninter_w = ninter;
     for (int o = 16; o > 0; o >>= 1) {
-        nstep += __shfl_down_sync(0xffffffffu, nstep, o);
-        npush += __shfl_down_sync(0xffffffffu, npush, o);
-        ninter += __shfl_down_sync(0xffffffffu, ninter, o);
+        nstep_w += __shfl_down_sync(0xffffffffu, nstep_w, o);
+        npush_w += __shfl_down_sync(0xffffffffu, npush_w, o);
+        ninter_w += __shfl_down_sync(0xffffffffu, ninter_w, o);
         edep_tot += __shfl_down_sync(0xffffffffu, edep_tot, o);
         esc_tot += __shfl_down_sync(0xffffffffu, esc_tot, o);
         if (SPLIT) nwide += __shfl_down_sync(0xffffffffu, nwide, o);
     }
     if (lane == 0) {
-        if (SPLIT) atomicAdd(P.counters + CNT_EWIDE, nwide);
-        atomicAdd(P.counters + CNT_ELANES, lanes);
-        atomicAdd(P.counters + CNT_EITER, iters);
-        atomicAdd(P.counters + CNT_ESTEP, nstep);
-        atomicAdd(P.counters + CNT_EPUSH, npush);
-        atomicAdd(P.counters + CNT_EINTER, ninter);
+        if (SPLIT) atomicAdd(P.counters + CNT_EWIDE, (unsigned long long)nwide);
+        atomicAdd(P.counters + CNT_ELANES, (unsigned long long)lanes);
+        atomicAdd(P.counters + CNT_EITER, (unsigned long long)iters);
+        atomicAdd(P.counters + CNT_ESTEP, nstep_w);
+        atomicAdd(P.counters + CNT_EPUSH, npush_w);
+        atomicAdd(P.counters + CNT_EINTER, ninter_w);
         atomicAdd(P.energy + 0, edep_tot);
         atomicAdd(P.energy + 1, esc_tot);
     }
