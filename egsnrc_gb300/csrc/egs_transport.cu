@@ -32,6 +32,7 @@
 #include <new>
 #include <mutex>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <type_traits>
 #include <vector>
@@ -1914,14 +1915,20 @@ static void fast_divisor(uint32_t d, uint32_t &m, int &l) {
 // host loops of the phantom uploads (tens of millions of voxels per step for
 // a caller that uploads its phantoms every time).
 template <class F>
-static void host_parallel(long long n, F f) {
+static void host_parallel(long long n, F f, long long small = 1LL << 20, long long grain = 1) {
     unsigned t = std::min(16u, std::max(1u, std::thread::hardware_concurrency()));
-    if (n < (1LL << 20) || t == 1) { f(0LL, n); return; }
+    t = (unsigned)std::min<long long>(t, n / grain);   // a thread costs about 30 us to start
+    if (n < small || t <= 1) { f(0LL, n); return; }
     std::vector<std::thread> th;
     const long long per = (n + t - 1) / t;
     for (unsigned k = 0; k < t; ++k) {
         const long long b = k * per, e = std::min(n, b + per);
-        if (b < e) th.emplace_back(f, b, e);
+        if (b >= e) break;
+        try {
+            th.emplace_back(f, b, e);
+        } catch (const std::system_error &) {   // no more threads: this one does the share
+            f(b, e);
+        }
     }
     for (auto &x : th) x.join();
 }
@@ -3525,28 +3532,56 @@ int egsgpu_get_phantom_info(egsgpu_handle *h, int k, long long *out) {
 
 }  // extern "C"
 
+// Writes arrays that a copy from the device is about to fill, over host threads:
+// arrays fresh from the allocator have no pages yet, and the copy takes them one
+// fault at a time (128^3 voxels: 10 ms).
+static void touch(double *a, double *b, long long n) {
+    host_parallel(n, [&](long long i, long long e) {
+        std::fill(a + i, a + e, 0.0);
+        if (b) std::fill(b + i, b + e, 0.0);
+    }, 1LL << 18, 1LL << 17);
+}
+
+// Batch sums (dose) and sums of squares (sigma, may be null) of N histories in
+// phantom G (the handle's or one of several) to dose and its standard deviation,
+// in place: the sums are read straight into the caller's arrays, without copies
+// the size of the phantom that would have to be paged in on each call.  Over
+// host threads from 2^15 voxels (dose() of 128^3 voxels: 11.5 -> 2.2
+// ms, of 64^3: 1.47 -> 0.67 ms; one thread takes 5 ns a voxel).
+template <class Phantom>
+static void sums_to_dose(const egsgpu_handle &h, const Phantom &G, double N, double *dose, double *sigma) {
+    const double nb = (double)h.nbatch;
+    const long long nxy = (long long)G.nx * G.ny;
+    host_parallel(nxy * G.nz, [&](long long b, long long e) {
+        int iz = (int)(b / nxy), rr = (int)(b - iz * nxy), iy = rr / G.nx, ix = rr - iy * G.nx;
+        for (long long i = b; i < e; ++i) {
+            double vol = (G.xb[ix + 1] - G.xb[ix]) * (G.yb[iy + 1] - G.yb[iy]) * (G.zb[iz + 1] - G.zb[iz]);
+            double mass = vol * G.rhor[i] * h.H.media[G.med[i]].rho;
+            double norm = N > 0 ? 1.602e-10 / (mass * N) : 0;   // egs_dose_scoring.cpp:318-319
+            const double s = dose[i];
+            dose[i] = s * norm;
+            if (sigma) {
+                // batch method: sigma of the mean of nb batch totals
+                double mean = s / nb, var = nb > 1 ? (sigma[i] / nb - mean * mean) / (nb - 1) : 0;
+                sigma[i] = (var > 0 ? std::sqrt(var) * nb : 0) * norm;
+            }
+            if (++ix == G.nx) {
+                ix = 0;
+                if (++iy == G.ny) { iy = 0; ++iz; }
+            }
+        }
+    }, 1LL << 15, 1LL << 15);
+}
+
 extern "C" {
 
 int egsgpu_get_phantom_dose(egsgpu_handle *h, int k, double *dose, double *sigma) {
     if (!h || !dose || k < 0 || k >= (int)h->phantoms.size()) return EGSGPU_ERR_ARG;
     const auto &P = h->phantoms[k];
-    long long nv = (long long)P.nx * P.ny * P.nz;
-    std::vector<double> s(nv), s2(nv);
-    int rc = h->eng->read_sums(P.voff, nv, s.data(), s2.data(), h->err);
-    if (rc) return rc;
-    const double N = (double)P.nhist, nb = (double)h->nbatch;
-    for (long long i = 0; i < nv; ++i) {
-        int iz = (int)(i / ((long long)P.nx * P.ny)), rr = (int)(i - (long long)iz * P.nx * P.ny);
-        int iy = rr / P.nx, ix = rr - iy * P.nx;
-        double vol = (P.xb[ix + 1] - P.xb[ix]) * (P.yb[iy + 1] - P.yb[iy]) * (P.zb[iz + 1] - P.zb[iz]);
-        double mass = vol * P.rhor[i] * h->H.media[P.med[i]].rho;
-        double norm = N > 0 ? 1.602e-10 / (mass * N) : 0;   // egs_dose_scoring.cpp:318-319
-        dose[i] = s[i] * norm;
-        if (sigma) {
-            double mean = s[i] / nb, var = nb > 1 ? (s2[i] / nb - mean * mean) / (nb - 1) : 0;
-            sigma[i] = (var > 0 ? std::sqrt(var) * nb : 0) * norm;
-        }
-    }
+    const long long nv = (long long)P.nx * P.ny * P.nz;
+    touch(dose, sigma, nv);
+    if (int rc = h->eng->read_sums(P.voff, nv, dose, sigma, h->err)) return rc;
+    sums_to_dose(*h, P, (double)P.nhist, dose, sigma);
     return 0;
 }
 
@@ -3573,24 +3608,9 @@ int egsgpu_get_tallies(egsgpu_handle *h, double *sum, double *sum2, double *tota
 int egsgpu_get_dose(egsgpu_handle *h, double *dose, double *sigma) {
     if (!h || !h->have_geom || !dose) return EGSGPU_ERR_ARG;
     if (h->multi()) { h->err = "several phantoms are set: use egsgpu_get_phantom_dose"; return EGSGPU_ERR_STATE; }
-    long long nv = h->nvox();
-    std::vector<double> s(nv), s2(nv);
-    int rc = egsgpu_get_tallies(h, s.data(), s2.data(), nullptr);
-    if (rc) return rc;
-    const double N = (double)h->nhist, nb = (double)h->nbatch;
-    for (long long i = 0; i < nv; ++i) {
-        int iz = (int)(i / ((long long)h->nx * h->ny)), rr = (int)(i - (long long)iz * h->nx * h->ny);
-        int iy = rr / h->nx, ix = rr - iy * h->nx;
-        double vol = (h->xb[ix + 1] - h->xb[ix]) * (h->yb[iy + 1] - h->yb[iy]) * (h->zb[iz + 1] - h->zb[iz]);
-        double mass = vol * h->rhor[i] * h->H.media[h->med[i]].rho;
-        double norm = N > 0 ? 1.602e-10 / (mass * N) : 0;   // egs_dose_scoring.cpp:318-319
-        dose[i] = s[i] * norm;
-        if (sigma) {
-            // batch method: sigma of the mean of nb batch totals
-            double mean = s[i] / nb, var = nb > 1 ? (s2[i] / nb - mean * mean) / (nb - 1) : 0;
-            sigma[i] = (var > 0 ? std::sqrt(var) * nb : 0) * norm;
-        }
-    }
+    touch(dose, sigma, h->nvox());
+    if (int rc = h->eng->read_sums(0, h->nvox(), dose, sigma, h->err)) return rc;
+    sums_to_dose(*h, *h, (double)h->nhist, dose, sigma);
     return 0;
 }
 
