@@ -60,7 +60,7 @@ struct Tables {
     const Real *shell;    // [shell_off + i][4]: eno (alias threshold), be (rm units), Jo, erfJo
     const int *shell_at;  // [shell_off + i]: alias bin (1-based)
     const Real *elem;     // [elem_off + k][96]: edge_a[16] b[16] c[16] d[16] energies[16] binding[6] iprob[6] | nedge
-    const Real *ms;       // [MS_NL*MS_NQ*MS_NU][3]: ums, fms, wms
+    const Real *ms;       // [MS_NL*MS_NQ*MS_NU][4]: ums, fms, wms, ums of the next bin - ums
     const int *ms_i;      // [MS_NL*MS_NQ*MS_NU]
     Real dllambi, dqmsi;
     int nmed;
@@ -307,6 +307,19 @@ struct RngLocal {
         return ((float)(x >> 9) + 0.5f) * (1.0f / 8388608.0f);
     }
 };
+// Reads of tables and geometry, which no kernel writes: the compiler may keep the
+// value or read it early, across atomics and warp joins.  Quadruples are aligned
+// to their size (16 bytes at most in one access).
+template <class T> __device__ inline T ldg(const T *p) { return __ldg(p); }
+template <class Real> struct Quad { Real x, y, z, w; };
+__device__ inline Quad<float> ldg4(const float *p) {
+    const float4 v = __ldg(reinterpret_cast<const float4 *>(p));
+    return {v.x, v.y, v.z, v.w};
+}
+__device__ inline Quad<double> ldg4(const double *p) {
+    const double2 a = __ldg(reinterpret_cast<const double2 *>(p)), b = __ldg(reinterpret_cast<const double2 *>(p) + 1);
+    return {a.x, a.y, b.x, b.y};
+}
 // Uniform in (0,1) with 23 random bits: the same value in FP32 and FP64.
 template <class Real, class R>
 __device__ inline Real urand(R &r) { return (Real)r.u(); }

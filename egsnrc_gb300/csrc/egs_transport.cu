@@ -2260,7 +2260,8 @@ struct Engine : EngineBase {
             loff += m.nne;
         }
         for (size_t i = 0; i < H.ums.size(); ++i) {
-            ms.push_back((Real)H.ums[i]); ms.push_back((Real)H.fms[i]); ms.push_back((Real)H.wms[i]);
+            const Real u = (Real)H.ums[i], un = i + 1 < H.ums.size() ? (Real)H.ums[i + 1] : u;
+            ms.push_back(u); ms.push_back((Real)H.fms[i]); ms.push_back((Real)H.wms[i]); ms.push_back(un - u);
             msi.push_back(H.ims[i]);
         }
         auto up = [&](DevMem &d, const void *src, size_t bytes) -> cudaError_t {
