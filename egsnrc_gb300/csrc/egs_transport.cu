@@ -885,9 +885,8 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 ? 8 : 1) k_photon
         }
         // :PTRANS: one voxel
         if (++s.nsteps > STEP_CAP) { err = 1; alive = false; continue; }
-        Real gmfp = s.gmfpr0 / s.rhor * s.cohfac;
-        Real ustep = gmfp * s.dpmfp;
         if (HFL) {
+            const Real ustep = s.gmfpr0 / s.rhor * s.cohfac * s.dpmfp;
             ++nstep;
             if (hfl_dist_out(G, p) <= ustep) { esc_tot += (double)(p.E * p.wt); alive = false; continue; }
             p.x += p.u * ustep; p.y += p.v * ustep; p.z += p.w * ustep;
@@ -896,23 +895,61 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 ? 8 : 1) k_photon
             s.state = 3;
             continue;
         }
+        // The voxel walk of EGS_XYZGeometry::howfar (see howfar), with what a flight
+        // does not change taken out of the loop: the voxel's decoding (jx, jy, jz are
+        // the next planes' indices).  The voxel entered is read while the distances
+        // to its faces are computed.  The walk is two thirds of this kernel's time
+        // and bound by its dependent chain and by issue; decoding the index, choosing
+        // the planes and waiting for the medium at every voxel cost 30% of it
+        // (one GB300: slab64 1e8 histories 488 -> 444 ms, 2e6 18.3 -> 17.2 ms, 512
+        // noalloc 1.54 -> 1.48 ms).
+        const Geom<Real> &GP = geom_of<Real, Multi>(P, p.pb);
+        const Real *xb = GP.xb, *yb = GP.yb, *zb = GP.zb;
+        int jx, jy, jz;
+        {
+            const int loc = p.ir - GP.voff;
+            jz = fdiv(loc, GP.mnxy, GP.lnxy);
+            const int r = loc - jz * GP.nxy;
+            jy = fdiv(r, GP.mnx, GP.lnx);
+            jx = r - jy * GP.nx + (p.u > 0);
+            jy += p.v > 0;
+            jz += p.w > 0;
+        }
+        int mnew = s.medium;
 #pragma unroll 1
-        for (int hop = 0;; ++hop) {
-            if (hop) { gmfp = s.gmfpr0 / s.rhor * s.cohfac; ustep = gmfp * s.dpmfp; }
-            int irnew = howfar(geom_of<Real, Multi>(P, p.pb), p.ir, p.x, p.y, p.z, p.u, p.v, p.w, ustep);
+        for (int hop = 1;; ++hop) {
+            const Real dx = (ldg(xb + jx) - p.x) / p.u, dy = (ldg(yb + jy) - p.y) / p.v,
+                       dz = (ldg(zb + jz) - p.z) / p.w;   // (unused along an axis the photon does not move)
+            if (mnew != s.medium) { s.medium = mnew; s.state = 1; break; }
+            const Real gmfp = s.gmfpr0 / s.rhor * s.cohfac;
+            Real ustep = gmfp * s.dpmfp;
+            int axis = -1;
+            if (p.u != 0 && dx <= ustep) { ustep = (dx <= GP.bt) ? GP.hbt : dx; axis = 0; }
+            if (p.v != 0 && dy <= ustep) { ustep = (dy <= GP.bt) ? GP.hbt : dy; axis = 1; }
+            if (p.w != 0 && dz <= ustep) { ustep = (dz <= GP.bt) ? GP.hbt : dz; axis = 2; }
             ++nstep;
             if (Adj) gadd(P, ga, p.ir, -Gh * (ustep / gmfp) / s.rhor);
             p.x += p.u * ustep; p.y += p.v * ustep; p.z += p.w * ustep;
             s.dpmfp = dmax((Real)0, s.dpmfp - ustep / gmfp);
-            if (irnew != p.ir) {
-                p.ir = irnew;
-                if (irnew < 0) { esc_tot += (double)(p.E * p.wt); alive = false; break; }
-                int mnew = G.med[irnew];
-                s.rhor = G.rhor[irnew];
-                if (mnew != s.medium) { s.medium = mnew; s.state = 1; break; }
+            if (axis >= 0) {
+                bool out;
+                if (axis == 0) {
+                    if (p.u > 0) { out = jx >= GP.nx; ++jx; ++p.ir; } else { --jx; out = jx < 0; --p.ir; }
+                } else if (axis == 1) {
+                    if (p.v > 0) { out = jy >= GP.ny; ++jy; p.ir += GP.nx; } else { --jy; out = jy < 0; p.ir -= GP.nx; }
+                } else {
+                    if (p.w > 0) { out = jz >= GP.nz; ++jz; p.ir += GP.nxy; } else { --jz; out = jz < 0; p.ir -= GP.nxy; }
+                }
+                if (out) { p.ir = -1; esc_tot += (double)(p.E * p.wt); alive = false; break; }
+                mnew = ldg(G.med + p.ir);
+                s.rhor = ldg(G.rhor + p.ir);
             }
-            if (!(s.dpmfp > (Real)1e-8)) { s.state = 3; break; }
-            if (hop + 1 >= PHOTON_HOPS || ++s.nsteps > STEP_CAP) break;
+            const bool due = !(s.dpmfp > (Real)1e-8);
+            if (due || hop >= PHOTON_HOPS || ++s.nsteps > STEP_CAP) {
+                if (mnew != s.medium) { s.medium = mnew; s.state = 1; }
+                else if (due) s.state = 3;
+                break;
+            }
         }
     }
     acc_flush(P, acc);
