@@ -160,8 +160,8 @@ __host__ __device__ inline uint64_t child_sid(uint64_t sid, uint32_t n, uint32_t
 static __host__ __device__ __noinline__ uint4 philox_block(uint32_t b, uint32_t s0, uint32_t s1, uint32_t k0,
                                                            uint32_t k1);
 
-// The generator keeps a window of the stream's next four Philox blocks
-// (number i in word i & 15; `lim` is one past the highest number held).  A
+// The generator keeps a window of the stream's next W numbers (W / 4 Philox
+// blocks; number i in word i & (W - 1); `lim` is one past the highest held).  A
 // draw computes only a block that is missing.  The transport loops call
 // ahead(k) where the warp is converged, so that the blocks the lanes will
 // need for the coming step are computed there, by all lanes together, instead
@@ -184,23 +184,25 @@ static __host__ __device__ __noinline__ uint4 philox_block(uint32_t b, uint32_t 
 // first must drop() its window before it draws again.
 constexpr int RNG_THREADS = 128;   // most threads of a CTA whose threads draw
 #ifdef __CUDA_ARCH__
+template <int W>
 __device__ inline uint32_t *rng_window() {
-    __shared__ uint32_t w[16 * RNG_THREADS];
+    __shared__ uint32_t w[W * RNG_THREADS];
     return w + threadIdx.x;
 }
 #endif
-struct Rng {
+template <int W>
+struct RngW {
     uint32_t seed, hist, n, lim;
     uint64_t sid;
 #ifdef __CUDA_ARCH__
-    __device__ inline uint32_t &word(uint32_t i) { return rng_window()[i * RNG_THREADS]; }
+    __device__ inline uint32_t &word(uint32_t i) { return rng_window<W>()[i * RNG_THREADS]; }
 #else
-    uint32_t c[16];
+    uint32_t c[W];
     uint32_t &word(uint32_t i) { return c[i]; }
 #endif
-    Rng() = default;
-    __host__ __device__ Rng(const Rng &o) : seed(o.seed), hist(o.hist), n(o.n), lim(0), sid(o.sid) {}
-    __host__ __device__ Rng &operator=(const Rng &o) {
+    RngW() = default;
+    __host__ __device__ RngW(const RngW &o) : seed(o.seed), hist(o.hist), n(o.n), lim(0), sid(o.sid) {}
+    __host__ __device__ RngW &operator=(const RngW &o) {
         seed = o.seed; hist = o.hist; n = o.n; sid = o.sid; lim = 0;
         return *this;
     }
@@ -209,7 +211,7 @@ struct Rng {
     }
     __host__ __device__ inline void drop() { lim = 0; }
     __host__ __device__ inline void put(uint32_t b, uint32_t o0, uint32_t o1, uint32_t o2, uint32_t o3) {
-        const uint32_t w = (b & 3u) << 2;
+        const uint32_t w = (b << 2) & (W - 1);
         word(w) = o0; word(w + 1) = o1; word(w + 2) = o2; word(w + 3) = o3;
     }
     __host__ __device__ inline void fill(uint32_t b) {
@@ -217,7 +219,7 @@ struct Rng {
         put(b, o.x, o.y, o.z, o.w);
         lim = (b << 2) + 4;
     }
-    // make the blocks holding the next k numbers (1 <= k <= 13) present.  The ten
+    // make the blocks holding the next k numbers (1 <= k <= W - 3) present.  The ten
     // rounds are inlined here (one copy per transport loop): a call to the
     // shared out-of-line block from this site measured 10-20% slower.
     __host__ __device__ inline void ahead(uint32_t k) {
@@ -236,10 +238,10 @@ struct Rng {
         return make_float2(a, draw());
     }
     __host__ __device__ inline float draw() {
-        // present: n < lim, and n >= lim - 16 since ahead() never runs more
-        // than three blocks past the current one
+        // present: n < lim, and n >= lim - W since ahead() never runs further than
+        // W / 4 - 1 blocks past the current one
         if (n >= lim) fill(n >> 2);
-        const uint32_t x = word(n & 15u);
+        const uint32_t x = word(n & (W - 1));
         ++n;
         // (x >> 9) + 0.5 scaled by 2^-23: exact in FP32 and FP64, in (0,1).  The
         // fused form has the same value and cannot be fused again into the
@@ -251,6 +253,7 @@ struct Rng {
 #endif
     }
 };
+using Rng = RngW<16>;
 // The same generator with its window in the object, so in local memory, and
 // its draws out of line: for the source kernel, and for the kernels whose own
 // state leaves no registers for the position and key (HOWFARLESS, the precision
@@ -258,7 +261,7 @@ struct Rng {
 struct RngLocal {
     uint32_t seed, hist, n, next;
     uint64_t sid;
-    alignas(16) uint32_t c[16];
+    alignas(16) uint32_t c[32];
     RngLocal() = default;
     __host__ __device__ RngLocal(const RngLocal &o) : seed(o.seed), hist(o.hist), n(o.n), next(0), sid(o.sid) {}
     __host__ __device__ RngLocal &operator=(const RngLocal &o) {
@@ -269,10 +272,10 @@ struct RngLocal {
         seed = s; hist = h; sid = id; n = n0; next = 0;
     }
     __host__ __device__ inline void fill(uint32_t b) {
-        reinterpret_cast<uint4 *>(c)[b & 3u] = philox_block(b, (uint32_t)sid, (uint32_t)(sid >> 32), seed, hist);
+        reinterpret_cast<uint4 *>(c)[b & 7u] = philox_block(b, (uint32_t)sid, (uint32_t)(sid >> 32), seed, hist);
     }
     __host__ __device__ inline void drop() { next = 0; }
-    // make the blocks holding the next k numbers (1 <= k <= 13) present.  The ten
+    // make the blocks holding the next k numbers (1 <= k <= 29) present.  The ten
     // rounds are inlined here (one copy per transport loop): a call to the
     // shared out-of-line block from this site measured 10-20% slower.
     __host__ __device__ inline void ahead(uint32_t k) {
@@ -281,7 +284,7 @@ struct RngLocal {
         for (; b <= b1; ++b) {
             uint32_t o[4];
             philox10(b, (uint32_t)sid, (uint32_t)(sid >> 32), 0u, seed, hist, o);
-            reinterpret_cast<uint4 *>(c)[b & 3u] = make_uint4(o[0], o[1], o[2], o[3]);
+            reinterpret_cast<uint4 *>(c)[b & 7u] = make_uint4(o[0], o[1], o[2], o[3]);
         }
         if (b > next) next = b;
     }
@@ -298,10 +301,10 @@ struct RngLocal {
     }
     __host__ __device__ inline float draw() {
         const uint32_t b = n >> 2;
-        // present: b < next, and b >= next - 4 since ahead() never runs more
-        // than three blocks past the current one
+        // present: b < next, and b >= next - 8 since ahead() never runs more
+        // than seven blocks past the current one
         if (b >= next) { fill(b); next = b + 1; }
-        const uint32_t x = c[n & 15u];
+        const uint32_t x = c[n & 31u];
         ++n;
         // (x >> 9) + 0.5 scaled by 2^-23: exact in FP32 and FP64, in (0,1)
         return ((float)(x >> 9) + 0.5f) * (1.0f / 8388608.0f);

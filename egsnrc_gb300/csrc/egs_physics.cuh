@@ -29,9 +29,9 @@ struct AzimDraw {
     uint32_t n, lim;
     int err;
 };
-template <class Real>
+template <class Real, int W>
 __device__ __noinline__ AzimDraw<Real> azimuth_draw(uint32_t n, uint32_t lim, uint32_t seed, uint32_t hist, uint64_t sid) {
-    Rng r;
+    RngW<W> r;
     r.n = n; r.lim = lim; r.seed = seed; r.hist = hist; r.sid = sid;
     Real xphi, xphi2, yphi, yphi2, rho2;
     int it = 0, err = 0;
@@ -45,9 +45,9 @@ __device__ __noinline__ AzimDraw<Real> azimuth_draw(uint32_t n, uint32_t lim, ui
     rho2 = 1 / rho2;
     return {(xphi2 - yphi2) * rho2, 2 * xphi * yphi * rho2, r.n, r.lim, err};
 }
-template <class Real>
-__device__ inline Azim<Real> azimuth(Rng &r, int &err) {
-    const AzimDraw<Real> a = azimuth_draw<Real>(r.n, r.lim, r.seed, r.hist, r.sid);
+template <class Real, int W>
+__device__ inline Azim<Real> azimuth(RngW<W> &r, int &err) {
+    const AzimDraw<Real> a = azimuth_draw<Real, W>(r.n, r.lim, r.seed, r.hist, r.sid);
     r.n = a.n;
     r.lim = a.lim;
     err |= a.err;
@@ -95,7 +95,7 @@ __device__ inline void rayleigh(const Tables<Real> &T, int med, Real E, Real gle
     const Real *xg = T.ray + (size_t)med * 4 * NRAY, *fc = xg + NRAY, *ba = fc + NRAY, *ca = ba + NRAY;
     const int *ia = T.ray_i + (size_t)med * NRAY;
     Real pmax = pm[1] * gle + pm[0], xmax = hc_i * E, xv, csq, rn1;
-    constexpr bool own = std::is_same<R, Rng>::value;   // written-out rounding (RngLocal: the compiler's)
+    constexpr bool own = !std::is_same<R, RngLocal>::value;   // written-out rounding (RngLocal: the compiler's)
     int it = 0;
     do {
         rn1 = urand<Real>(r);

@@ -135,6 +135,13 @@ constexpr int INTER_MAXWAIT = 24;   // longest wait of a lane due to interact
 // deflections, two azimuths, the lateral displacement), plus one for a new
 // step length and one for the fictitious-cross-section test.
 constexpr unsigned RNG_AHEAD = 13;
+// With small path lengths (at most 13.8 elastic mean free paths) a step takes two
+// more, and each rejected azimuth another two, so in most iterations some lane ran
+// past 13 and the warp computed a block for it alone.  20 numbers in a window of
+// 32, one GB300, 13 -> 16 -> 20 -> 28 numbers: slab64 1e8 443 -> 429 -> 420 -> 423
+// ms, water30 1e6 25.0 -> 23.9 -> 23.5 -> 23.5 ms, water128e 2e5 117.6 -> 115.8 ->
+// 113.8 -> 116.0 ms; HOWFARLESS (local window) 1e6 110.1 -> 106.8 ms at 20.
+constexpr unsigned RNG_AHEAD_STEP = 20;
 constexpr int MAX_BLOCK = RNG_THREADS;   // launch bound of the transport kernels (threads per CTA)
 constexpr double VERY_FAR = 1e30;   // egs++ veryFar (egs++/egs_functions.h:105)
 // Distance to a voxel face (cm) within which an FP32 electron step is computed
@@ -1157,7 +1164,7 @@ __device__ __noinline__ Real wide_eloss(const Tables<Real> &T, const MedScalars<
 // joins only before the hinge: measured no faster otherwise.
 template <class Real, bool Multi, bool Adj = false, bool HFL = false, bool PI = false, bool SPL = false>
 __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL || SPL ? 6 : 5) : 1) k_electron(Params<Real> P) {
-    using R = typename std::conditional<Adj || HFL || SPL, RngLocal, Rng>::type;
+    using R = typename std::conditional<Adj || HFL || SPL, RngLocal, RngW<32>>::type;
     const Tables<Real> &T = P.T;
     const Geom<Real> &G = P.G;
     const unsigned lane = threadIdx.x & 31u;
@@ -1271,7 +1278,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL ||
         ++iters;
         // the random-number blocks of the coming step, computed by the warp's
         // live lanes together (Rng::ahead)
-        if (alive) p.rng.ahead(RNG_AHEAD);
+        if (alive) p.rng.ahead(RNG_AHEAD_STEP);
         // Discrete interactions are sampled for several lanes at once (see the
         // photon kernel): inter_batch of 32 live lanes, and the same share of
         // fewer, so that the few lanes left in a launch's tail do not wait for
