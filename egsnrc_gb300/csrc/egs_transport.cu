@@ -128,7 +128,8 @@ constexpr unsigned REQUEUE_MIN = 32768;
 constexpr int LSTACK = 6;   // per-thread LIFO depth for charged secondaries
 // A photon lane crosses up to this many voxels per iteration of the persistent
 // loop before the warp's bookkeeping (refill, interaction batching) runs again.
-constexpr int PHOTON_HOPS = 16;
+// 10, 12, 16, 24, 32 crossings: slab64 1e8 412, 409, 413, 413, 422 ms.
+constexpr int PHOTON_HOPS = 12;
 constexpr int INTER_MAXWAIT = 24;   // longest wait of a lane due to interact
 // Random numbers made present ahead of an electron step or an interaction
 // batch: a PRESTA-II step with the q-surface sampler takes 11 (two
