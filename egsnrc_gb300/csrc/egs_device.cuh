@@ -232,25 +232,47 @@ struct RngW {
         }
         if ((b << 2) > lim) lim = b << 2;
     }
-    __host__ __device__ inline float u() { return draw(); }
-    __host__ __device__ inline float2 u2() {
-        float a = draw();
-        return make_float2(a, draw());
-    }
-    __host__ __device__ inline float draw() {
-        // present: n < lim, and n >= lim - W since ahead() never runs further than
-        // W / 4 - 1 blocks past the current one
-        if (n >= lim) fill(n >> 2);
+    // The next number, known to be present: after ahead(k) or ensure(k) for k draws.
+    // A draw that checks costs more than its check: the lanes that take its slow
+    // path leave the others, and the code behind it runs once for each group.  With
+    // one check for a pair, none in the step's straight-line draws and no integer
+    // conversion, one GB300: slab64 1e8 409 -> 363 ms, water30 1e6 23.4 -> 20.0 ms,
+    // water128e 2e5 114 -> 101 ms, perturbed64 32.1 -> 28.7 ms, noalloc 512 1.46 ->
+    // 1.38 ms.
+    __host__ __device__ inline float get() {
         const uint32_t x = word(n & (W - 1));
         ++n;
-        // (x >> 9) + 0.5 scaled by 2^-23: exact in FP32 and FP64, in (0,1).  The
-        // fused form has the same value and cannot be fused again into the
-        // caller's expression, whose rounding must not depend on inlining.
+        // (x >> 9) + 0.5 scaled by 2^-23: exact in FP32 and FP64, in (0,1).  On the
+        // device as 1.(x >> 9) - (1 - 2^-24), the same value without a conversion;
+        // an addition cannot be fused into the caller's expression, whose rounding
+        // must not depend on inlining.
 #ifdef __CUDA_ARCH__
-        return __fmaf_rn((float)(x >> 9), 1.0f / 8388608.0f, 1.0f / 16777216.0f);
+        return __fadd_rn(__uint_as_float(__funnelshift_r(x, 0x7fu, 9)), -(1.0f - 1.0f / 16777216.0f));
 #else
         return ((float)(x >> 9) + 0.5f) * (1.0f / 8388608.0f);
 #endif
+    }
+    __host__ __device__ inline float2 get2() {
+        const float a = get();
+        return make_float2(a, get());
+    }
+    // make the next k numbers (1 <= k <= W - 3) present where the lanes are apart
+    __host__ __device__ inline void ensure(uint32_t k) {
+        while (n + k > lim) fill((lim > n ? lim : n) >> 2);
+    }
+    __host__ __device__ inline float u() {
+        // present: n < lim, and n >= lim - W since ahead() never runs further than
+        // W / 4 - 1 blocks past the current one
+        if (n >= lim) fill(n >> 2);
+        return get();
+    }
+    // two consecutive numbers with one check
+    __host__ __device__ inline float2 u2() {
+        if (n + 2 > lim) {
+            if (n >= lim) fill(n >> 2);
+            if (n + 2 > lim) fill(lim >> 2);
+        }
+        return get2();
     }
 };
 using Rng = RngW<16>;
@@ -275,6 +297,10 @@ struct RngLocal {
         reinterpret_cast<uint4 *>(c)[b & 7u] = philox_block(b, (uint32_t)sid, (uint32_t)(sid >> 32), seed, hist);
     }
     __host__ __device__ inline void drop() { next = 0; }
+    // (its draws check by themselves)
+    __host__ __device__ inline float get() { return u(); }
+    __host__ __device__ inline float2 get2() { return u2(); }
+    __host__ __device__ inline void ensure(uint32_t) {}
     // make the blocks holding the next k numbers (1 <= k <= 29) present.  The ten
     // rounds are inlined here (one copy per transport loop): a call to the
     // shared out-of-line block from this site measured 10-20% slower.

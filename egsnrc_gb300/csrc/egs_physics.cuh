@@ -437,16 +437,19 @@ __device__ inline void pair(const MedScalars<Real> &M, Particle<Real, R> &p, Rea
 template <class Real>
 struct MsState { bool find_index; int i, j; Real omega2; };
 
-// mscat, spin effects off (src/egsnrc.mortran:2984-3136)
+// mscat, spin effects off (src/egsnrc.mortran:2984-3136).  The caller has made
+// MSCAT_DRAWS numbers present, the most it takes; only the short-path loop, which
+// may take more, checks its draws.
+constexpr unsigned MSCAT_DRAWS = 5;
 template <class Real, class R>
 __device__ inline void mscat(const Tables<Real> &T, R &r, Real lambda, Real chia2, Real q1, MsState<Real> &st,
                              Real &cost, Real &sint, int &err) {
     if (lambda <= (Real)13.8) {
-        Real sprob = urand<Real>(r), explambda = dexp(-lambda);
+        Real sprob = (Real)r.get(), explambda = dexp(-lambda);
         if (sprob < explambda) { cost = 1; sint = 0; return; }
         Real wsum = (1 + lambda) * explambda;
         if (sprob < wsum) {
-            Real xi = urand<Real>(r);
+            Real xi = (Real)r.get();
             xi = 2 * chia2 * xi / (1 - xi + chia2);
             cost = 1 - xi;
             sint = dsqrt(xi * (2 - xi));
@@ -484,7 +487,7 @@ __device__ inline void mscat(const Tables<Real> &T, R &r, Real lambda, Real chia
             ai -= i;
             const bool drawj = !(q1 < (Real)1e-3) && q1 < (Real)0.5;
             float2 qij;
-            if (drawj) qij = urand2(r); else qij = make_float2(r.u(), 0.f);
+            if (drawj) qij = r.get2(); else qij = make_float2(r.get(), 0.f);
             Real xi = (Real)qij.x;
             if (xi < ai) ++i;
             i = min(max(i, 0), MS_NL - 1);
@@ -506,7 +509,7 @@ __device__ inline void mscat(const Tables<Real> &T, R &r, Real lambda, Real chia
             st.i = i; st.j = j;
             st.find_index = false;
         }
-        const float2 qku = urand2(r);
+        const float2 qku = r.get2();
         Real xi = (Real)qku.x;
         Real ak = xi * (MS_NU - 1);
         int k = (int)ak;
@@ -567,6 +570,7 @@ __device__ inline void msdist_pII(const Tables<Real> &T, const MedScalars<Real> 
 #pragma unroll 1
     for (int half = 0; half < 2; ++half) {
         Real wh, sh;
+        p.rng.ensure(MSCAT_DRAWS);   // (the first azimuth may have run past the step's numbers)
         mscat(T, p.rng, lambda, chia2, xi, st, wh, sh, err);
         __syncwarp(lanes);
         Azim<Real> ah = azimuth<Real>(p.rng, err);

@@ -840,7 +840,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 ? 8 : 1) k_photon
                 if (Adj) gadd(P, ga, p.ir, Gh / s.rhor);
                 const MedScalars<Real> &M = cmed<Real>(s.medium);
                 const Real *g = T.gtab + ((size_t)M.gtab_off + s.lgle - 1) * 8;
-                Real r37 = urand<Real>(p.rng);
+                Real r37 = (Real)p.rng.get();
                 if (r37 <= 1 - s.cohfac) {   // Rayleigh (src/egsnrc.macros:1602-1613)
                     Real costhe, sinthe;
                     rayleigh(T, s.medium, p.E, s.gle, s.lgle, p.rng, costhe, sinthe, err);
@@ -1320,7 +1320,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL ||
                     bool brems = false;
                     if (p.iq < 0) {
                         Real ebr1 = rw[9] * s.elke + rw[8];
-                        Real r24 = urand<Real>(p.rng);
+                        Real r24 = (Real)p.rng.get();
                         brems = r24 <= ebr1;
                         if (!brems && p.E <= M2.thmoll) {
                             if (ebr1 <= 0) { s.state = 0; continue; }
@@ -1372,7 +1372,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL ||
                         }
                     } else {
                         Real pbr1 = rw[11] * s.elke + rw[10];
-                        Real r25 = urand<Real>(p.rng);
+                        Real r25 = (Real)p.rng.get();
                         if (r25 < pbr1) brems = true;
                         else {
                             Real pbr2 = rw[13] * s.elke + rw[12];
@@ -1550,7 +1550,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL ||
                 const MedScalars<Real> &M = cmed<Real>(s.medium);
                 s.compute_tstep = 1;
                 s.eke = p.E - rm;
-                Real r = urand<Real>(p.rng);
+                Real r = (Real)p.rng.get();   // (get: within the numbers made present above)
                 s.demfp = dmax(-dlog(r), (Real)1e-8);
                 s.elke = dlog(s.eke);
                 s.lelke = min(max((int)(M.eke1 * s.elke + M.eke0), 1), M.meke);
@@ -1646,7 +1646,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL ||
                 callhowfar = !(ustep < tperp);
             } else {
                 callmsdist = false;
-                Real rnnoss = urand<Real>(p.rng);
+                Real rnnoss = (Real)p.rng.get();
                 if (rnnoss < (Real)1e-30) rnnoss = (Real)1e-30;
                 Real lambda = -dlog(1 - rnnoss);
                 Real g1 = s.eke / rm + 1;
@@ -1728,7 +1728,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL ||
                         Real ekems = dmax(ekef, T.ecut - rm);
                         Real pp2 = ekems * (ekems + 2 * rm);
                         Real chia2 = M.xcc / (4 * M.blcc * pp2);
-                        Real xi = urand<Real>(p.rng);
+                        Real xi = (Real)p.rng.get();
                         xi = 2 * chia2 * xi / (1 - xi + chia2);
                         Real costhe = 1 - xi, sinthe = dsqrt(xi * (2 - xi));
                         Azim<Real> az = azimuth<Real>(p.rng, err);
