@@ -277,9 +277,8 @@ struct RngW {
 };
 using Rng = RngW<16>;
 // The same generator with its window in the object, so in local memory, and
-// its draws out of line: for the source kernel, and for the kernels whose own
-// state leaves no registers for the position and key (HOWFARLESS, the precision
-// split and the adjoint: with the shared window HOWFARLESS runs 8% slower).
+// its draws out of line: for the source kernel, which draws four numbers, and for
+// the precision split, whose FP32 rounding is not written out for other draws.
 struct RngLocal {
     uint32_t seed, hist, n, next;
     uint64_t sid;

@@ -2,8 +2,6 @@
 // (paths relative to HEN_HOUSE) and draws its random numbers from the
 // interacting particle's own Philox stream, in the reference's order.
 #pragma once
-#include <type_traits>
-
 #include "egs_device.cuh"
 
 namespace egsgpu {
@@ -87,7 +85,8 @@ __device__ inline void rotate(Real a, Real b, Real c, Real sinthe, Real costhe, 
 
 // ------------------------------------------------------------ Rayleigh ----
 // egs_rayleigh_sampling (src/egsnrc.mortran:8559-8590)
-template <class Real, class R>
+// FusedSin: the sine from 1 - cos^2 in one rounding, as the adjoint's replays have it
+template <bool FusedSin, class Real, class R>
 __device__ inline void rayleigh(const Tables<Real> &T, int med, Real E, Real gle, int lgle, R &r,
                                 Real &costhe, Real &sinthe, int &err) {
     const Real hc_i = (Real)80.65506856998, twice_hc2 = (Real)0.000307444456, dwi = (Real)(NRAY - 1);
@@ -95,13 +94,11 @@ __device__ inline void rayleigh(const Tables<Real> &T, int med, Real E, Real gle
     const Real *xg = T.ray + (size_t)med * 4 * NRAY, *fc = xg + NRAY, *ba = fc + NRAY, *ca = ba + NRAY;
     const int *ia = T.ray_i + (size_t)med * NRAY;
     Real pmax = pm[1] * gle + pm[0], xmax = hc_i * E, xv, csq, rn1;
-    constexpr bool own = !std::is_same<R, RngLocal>::value;   // written-out rounding (RngLocal: the compiler's)
     int it = 0;
     do {
         rn1 = urand<Real>(r);
         do {
-            const Real q = urand<Real>(r);
-            Real r0 = own ? rmul(q, pmax) : q * pmax;
+            Real r0 = rmul(urand<Real>(r), pmax);
             int ibin = 1 + (int)(r0 * dwi);
             int ib = ia[ibin - 1];
             if (ia[ibin] > ib) {
@@ -113,10 +110,10 @@ __device__ inline void rayleigh(const Tables<Real> &T, int med, Real E, Real gle
         } while (!(xv < xmax));
         xv = xv / E;
         costhe = 1 - twice_hc2 * xv * xv;
-        csq = own ? rmul(costhe, costhe) : costhe * costhe;
+        csq = rmul(costhe, costhe);
         if (it > LOOP_CAP) break;
     } while (!(2 * rn1 < 1 + csq));
-    sinthe = dsqrt(dmax((Real)0, 1 - csq));
+    sinthe = dsqrt(dmax((Real)0, FusedSin ? rfma(-costhe, costhe, (Real)1) : 1 - csq));
 }
 
 // ------------------------------------------------------------- Compton ----

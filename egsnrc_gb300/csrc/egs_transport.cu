@@ -141,7 +141,7 @@ constexpr unsigned RNG_AHEAD = 13;
 // past 13 and the warp computed a block for it alone.  20 numbers in a window of
 // 32, one GB300, 13 -> 16 -> 20 -> 28 numbers: slab64 1e8 443 -> 429 -> 420 -> 423
 // ms, water30 1e6 25.0 -> 23.9 -> 23.5 -> 23.5 ms, water128e 2e5 117.6 -> 115.8 ->
-// 113.8 -> 116.0 ms; HOWFARLESS (local window) 1e6 110.1 -> 106.8 ms at 20.
+// 113.8 -> 116.0 ms.
 constexpr unsigned RNG_AHEAD_STEP = 20;
 constexpr int MAX_BLOCK = RNG_THREADS;   // launch bound of the transport kernels (threads per CTA)
 constexpr double VERY_FAR = 1e30;   // egs++ veryFar (egs++/egs_functions.h:105)
@@ -550,12 +550,12 @@ __device__ int hfl_hinge(const Params<Real> &P, Acc<Real, Multi> &acc, const Geo
         return loc;
     }
     const Real d[3] = {p.x - xi0[0], p.y - xi0[1], p.z - xi0[2]};
-    const Real d2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+    const Real d2 = rfma(d[2], d[2], sum2(d[0], d[0], d[1], d[1]));
     Real t0 = tv, t1 = 0;
     Real u0[3] = {ui0[0], ui0[1], ui0[2]}, u1[3] = {0, 0, 0};
     if (ch_step) {
         if (urand<Real>(p.rng) < (Real)0.5) {   // hinge from the initial direction
-            Real c = 1 - (d[0] * u0[0] + d[1] * u0[1] + d[2] * u0[2]) / tv;
+            Real c = 1 - rfma(d[2], u0[2], sum2(d[0], u0[0], d[1], u0[1])) / tv;
             if (c < (Real)1e-3) {
                 t0 = dsqrt(d2);
                 for (int k = 0; k < 3; ++k) u0[k] = d[k] / t0;
@@ -566,7 +566,7 @@ __device__ int hfl_hinge(const Params<Real> &P, Acc<Real, Multi> &acc, const Geo
             }
         } else {                                 // hinge from the final direction
             u1[0] = p.u; u1[1] = p.v; u1[2] = p.w;
-            Real c = 1 - (d[0] * u1[0] + d[1] * u1[1] + d[2] * u1[2]) / tv;
+            Real c = 1 - rfma(d[2], u1[2], sum2(d[0], u1[0], d[1], u1[1])) / tv;
             if (c < (Real)1e-3) {
                 t0 = dsqrt(d2);
                 for (int k = 0; k < 3; ++k) u0[k] = d[k] / t0;
@@ -743,14 +743,13 @@ struct PhotonState {
 // would spill ~1 KB per thread at that bound and keeps its registers.
 template <class Real, bool Multi, bool Adj = false, bool HFL = false>
 __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 ? 8 : 1) k_photon(Params<Real> P) {
-    using R = typename std::conditional<Adj || HFL, RngLocal, Rng>::type;
     const Tables<Real> &T = P.T;
     const Geom<Real> &G = P.G;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned nq = *P.pin.count < P.pin.capacity ? *P.pin.count : P.pin.capacity;
     if (nq == 0) return;   // the queues have drained: the rounds enqueued past the last one
     if (threadIdx.x == 0 && blockIdx.x == 0) atomicMax(P.peak, *P.pin.count);
-    Particle<Real, R> p;
+    Particle<Real> p;
     PhotonState<Real> s;
     Acc<Real, Multi> acc{-1, 0u, (Real)0, 0u};
     AccG<Real> ga{-1, (Real)0};
@@ -763,7 +762,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 ? 8 : 1) k_photon
     const Real rm = (Real)RM;
     const bool requeue = P.requeue_lanes > 0 && nq >= REQUEUE_MIN;
     auto take = [&](unsigned idx) {   // queue record idx becomes this lane's particle
-        load_particle<Real, Multi, R>(P, P.pin, idx, p, acc);
+        load_particle<Real, Multi, Rng>(P, P.pin, idx, p, acc);
         if (Adj) Gh = hist_weight(P, p);
         alive = true;
         s.state = 0;
@@ -843,7 +842,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 ? 8 : 1) k_photon
                 Real r37 = (Real)p.rng.get();
                 if (r37 <= 1 - s.cohfac) {   // Rayleigh (src/egsnrc.macros:1602-1613)
                     Real costhe, sinthe;
-                    rayleigh(T, s.medium, p.E, s.gle, s.lgle, p.rng, costhe, sinthe, err);
+                    rayleigh<Adj>(T, s.medium, p.E, s.gle, s.lgle, p.rng, costhe, sinthe, err);
                     Azim<Real> az = azimuth<Real>(p.rng, err);
                     Real a = p.u, b = p.v, c = p.w;
                     rotate(a, b, c, sinthe, costhe, az, p.u, p.v, p.w);
@@ -856,7 +855,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 ? 8 : 1) k_photon
                     Real E2, u2, v2, w2;
                     int iq2;
                     pair(M, p, E2, iq2, u2, v2, w2, err);
-                    Particle<Real, R> q = p;
+                    Particle<Real> q = p;
                     q.E = E2; q.iq = iq2; q.u = u2; q.v = v2; q.w = w2;
                     q.rng.init(p.rng.seed, p.rng.hist, child_sid(p.rng.sid, p.rng.n, 0), 0u);
                     push_charged(P, P.ein, P.pout, p, acc, npush, edep_tot, err);
@@ -866,7 +865,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 ? 8 : 1) k_photon
                 }
                 Real gbr2 = g[5] * s.gle + g[4];
                 if (r36 < gbr2) {
-                    Particle<Real, R> e = p;
+                    Particle<Real> e = p;
                     Real edep = compton(T, M, p, e.u, e.v, e.w, e.E, err);
                     e.iq = -1;
                     e.rng.init(p.rng.seed, p.rng.hist, child_sid(p.rng.sid, p.rng.n, 0), 0u);
@@ -1177,11 +1176,11 @@ __device__ __noinline__ Real wide_eloss(const Tables<Real> &T, const MedScalars<
 // two thin groups.  FP32: five CTAs per SM, the most at which nothing spills
 // (94-96 registers; six were 80 with spills).  Both together, one GB300:
 // slab64 1e8 histories 526 -> 500 ms, water128e 2e5 163 -> 156 ms, perturbed64
-// 46.0 -> 40.8 ms.  HOWFARLESS and the precision split keep six, and HOWFARLESS
-// joins only before the hinge: measured no faster otherwise.
+// 46.0 -> 40.8 ms.  HOWFARLESS and the precision split keep six CTAs and only the
+// join before the deflection: measured no faster otherwise.
 template <class Real, bool Multi, bool Adj = false, bool HFL = false, bool PI = false, bool SPL = false>
 __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL || SPL ? 6 : 5) : 1) k_electron(Params<Real> P) {
-    using R = typename std::conditional<Adj || HFL || SPL, RngLocal, RngW<32>>::type;
+    using R = typename std::conditional<SPL, RngLocal, RngW<32>>::type;   // (see RngLocal)
     const Tables<Real> &T = P.T;
     const Geom<Real> &G = P.G;
     const unsigned lane = threadIdx.x & 31u;
