@@ -1169,7 +1169,7 @@ __device__ __noinline__ Real wide_eloss(const Tables<Real> &T, const MedScalars<
 // its own instantiation so that the default FP32 step carries none of it.
 //
 // The step is bound by the latency of its long dependent chains, not by issue
-// (53% of cycles) or memory.  The lanes that step carry their mask (`go`) and
+// (55% of cycles) or memory.  The lanes that step carry their mask (`go`) and
 // meet again after the start of a new step sequence, before the face distances
 // and after the deflection: left alone, the compiler threads the new sequences
 // past the join, and the warp ran the whole step 1.2-1.4 times per iteration in
@@ -1177,7 +1177,8 @@ __device__ __noinline__ Real wide_eloss(const Tables<Real> &T, const MedScalars<
 // (94-96 registers; six were 80 with spills).  Both together, one GB300:
 // slab64 1e8 histories 526 -> 500 ms, water128e 2e5 163 -> 156 ms, perturbed64
 // 46.0 -> 40.8 ms.  HOWFARLESS and the precision split keep six CTAs and only the
-// join before the deflection: measured no faster otherwise.
+// join before the deflection: measured no faster otherwise (HOWFARLESS 1e6 at
+// five 87.5 against 86.5 ms).
 template <class Real, bool Multi, bool Adj = false, bool HFL = false, bool PI = false, bool SPL = false>
 __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 && !Adj ? (HFL || SPL ? 6 : 5) : 1) k_electron(Params<Real> P) {
     using R = typename std::conditional<SPL, RngLocal, RngW<32>>::type;   // (see RngLocal)
