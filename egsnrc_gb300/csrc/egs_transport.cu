@@ -1971,6 +1971,7 @@ struct EngineBase {
     virtual int run_noalloc(const Source &S, long long first, long long n, uint32_t seed, double *dose,
                             cudaStream_t st, unsigned char *scratch, size_t scratch_bytes, std::string &err) = 0;
     virtual int problems(int n, const PhantomDesc *pd, const Source *src, std::string &err) = 0;
+    virtual int uploaded(std::string &err) = 0;   // after uploads made by the caller: runs wait for them
     virtual int run_multi(const Source &Smax, int nbatch, cudaStream_t st, std::string &err) = 0;
     virtual int adjoint(const Source &S, long long first, long long n, uint32_t seed, const double *w, double *grad,
                         std::string &err) = 0;
@@ -2101,6 +2102,18 @@ template <class Real>
 struct Engine : EngineBase {
     egsgpu_config cfg;
 
+    // Uploads and clearing go to the legacy default stream and return before they
+    // are done; the transport runs on streams that do not wait for that one (ws,
+    // or a non-blocking stream of the caller).  Every call that uploads or clears
+    // records this event behind its work, and every run waits for it on the device.
+    cudaEvent_t ev_up = nullptr;
+    int uploaded(std::string &err) override {
+        if (!ev_up) CK(cudaEventCreateWithFlags(&ev_up, cudaEventDisableTiming));
+        CK(cudaEventRecord(ev_up, cudaStreamLegacy));
+        return 0;
+    }
+    cudaError_t wait_uploads(cudaStream_t st) { return ev_up ? cudaStreamWaitEvent(st, ev_up, 0) : cudaSuccess; }
+
     int clear_tallies(long long nv, std::string &err) override {
         CK(cudaMemset(d_dose.p, 0, nv * dose_slots * sizeof(double)));
         CK(cudaMemset(d_sum.p, 0, nv * sizeof(double)));
@@ -2109,7 +2122,7 @@ struct Engine : EngineBase {
         CK(cudaMemset(d_counters.p, 0, CNT_N * sizeof(unsigned long long)));
         CK(cudaMemset(d_error.p, 0, 2 * sizeof(int)));
         for (int k = 0; k < 4; ++k) { prof_ms[k] = 0; prof_n[k] = 0; }
-        return 0;
+        return uploaded(err);
     }
     int read_sums(long long off, long long n, double *sum, double *sum2, std::string &err) override {
         if (sum) CK(cudaMemcpy(sum, (double *)d_sum.p + off, n * sizeof(double), cudaMemcpyDeviceToHost));
@@ -2128,7 +2141,7 @@ struct Engine : EngineBase {
         CK(cudaMemcpy(d_sum.p, sum, nv * sizeof(double), cudaMemcpyHostToDevice));
         CK(cudaMemcpy(d_sum2.p, sum2, nv * sizeof(double), cudaMemcpyHostToDevice));
         CK(cudaMemset(d_dose.p, 0, nv * dose_slots * sizeof(double)));
-        return 0;
+        return uploaded(err);
     }
     int read_profile(double *out, std::string &err) override {
         unsigned long long c[CNT_N];
@@ -2152,7 +2165,7 @@ struct Engine : EngineBase {
             CK(d_hist.alloc(n * sizeof(double)));
             CK(cudaMemset(d_hist.p, 0, n * sizeof(double)));
         }
-        return 0;
+        return uploaded(err);
     }
     int read_history_tally(double *out, std::string &err) override {
         if (hist_n > 0) CK(cudaMemcpy(out, d_hist.p, hist_n * sizeof(double), cudaMemcpyDeviceToHost));
@@ -2235,6 +2248,7 @@ struct Engine : EngineBase {
     ~Engine() {
         if (gexec) cudaGraphExecDestroy(gexec);
         if (gexec_loop) cudaGraphExecDestroy(gexec_loop);
+        if (ev_up) cudaEventDestroy(ev_up);
         if (events_ready) {
             for (auto &e : ev) cudaEventDestroy(e);
             for (auto &e : gev) cudaEventDestroy(e);
@@ -2359,7 +2373,7 @@ struct Engine : EngineBase {
         CK(cudaMemset(d_energy.p, 0, 2 * sizeof(double)));
         CK(cudaMemset(d_counters.p, 0, CNT_N * sizeof(unsigned long long)));
         CK(cudaMemset(d_error.p, 0, 2 * sizeof(int)));
-        return 0;
+        return uploaded(err);
     }
 
     // HOWFARLESS: the phantom must be one medium at one density; the step
@@ -2384,7 +2398,7 @@ struct Engine : EngineBase {
         CK(d_etab_hfl.alloc(e.size() * sizeof(Real)));
         CK(cudaMemcpy(d_etab_hfl.p, e.data(), e.size() * sizeof(Real), cudaMemcpyHostToDevice));
         hfl_mindel = mindel;
-        return 0;
+        return uploaded(err);
     }
 
     int geometry(int nx, int ny, int nz, const double *xb, const double *yb, const double *zb, const int32_t *med,
@@ -2432,7 +2446,7 @@ struct Engine : EngineBase {
         CK(cudaMemset(d_dose.p, 0, nvox * sizeof(double)));
         CK(cudaMemset(d_sum.p, 0, nvox * sizeof(double)));
         CK(cudaMemset(d_sum2.p, 0, nvox * sizeof(double)));
-        return 0;
+        return uploaded(err);
     }
 
     static constexpr size_t QUEUE_RECORD = 12 * sizeof(Real) + sizeof(int) + 2 * sizeof(int8_t) +
@@ -2670,7 +2684,8 @@ struct Engine : EngineBase {
         const long long groups = (nbatch + g - 1) / g;   // of even sizes
         return (int)((nbatch + groups - 1) / groups);
     }
-    // Room for `slots` batch slots; the new ones are cleared.
+    // Room for `slots` batch slots; the new ones are cleared, on the stream of the
+    // kernels that add to them (on another, the clearing could erase deposits).
     int ensure_slots(int &slots, std::string &err) {
         if (slots <= dose_slots) return 0;
         const size_t one = (size_t)nvox * sizeof(double), had = d_dose.n / one;
@@ -2681,11 +2696,12 @@ struct Engine : EngineBase {
                 slots = 1;
                 return 0;
             }
-            CK(cudaMemcpy(more.p, d_dose.p, one * dose_slots, cudaMemcpyDeviceToDevice));
+            CK(cudaMemcpyAsync(more.p, d_dose.p, one * dose_slots, cudaMemcpyDeviceToDevice, ws));
+            CK(cudaStreamSynchronize(ws));   // `more` takes the old array and frees it
             std::swap(more.p, d_dose.p);
             std::swap(more.n, d_dose.n);
         }
-        CK(cudaMemset((char *)d_dose.p + one * dose_slots, 0, one * (slots - dose_slots)));
+        CK(cudaMemsetAsync((char *)d_dose.p + one * dose_slots, 0, one * (slots - dose_slots), ws));
         dose_slots = slots;
         return 0;
     }
@@ -2726,7 +2742,6 @@ struct Engine : EngineBase {
         }
         int group = mode ? 1 : batches_per_group(total, nbatch, tune ? chunk : std::min(chunk, chunk0));
         if (cfg.use_graph > 0 && group < nbatch) group = 1;
-        if (int rc = ensure_slots(group, err)) return rc;
         // persistent grids, one per kernel: never more CTAs than can be
         // resident at once (the photon kernel, with fewer registers, fits more
         // CTAs per SM than the electron kernel)
@@ -2741,6 +2756,10 @@ struct Engine : EngineBase {
         }
         if (hfl)
             if (int rc = hfl_tables(err)) return rc;
+        CK(cudaEventRecord(ev_in, st));
+        CK(cudaStreamWaitEvent(ws, ev_in, 0));
+        CK(wait_uploads(ws));
+        if (int rc = ensure_slots(group, err)) return rc;
         // The launch shape of candidate k (see SHAPES): threads per CTA and the
         // grids of both kernels.
         int bs = 128, gp = 0, ge = 0;
@@ -2777,6 +2796,7 @@ struct Engine : EngineBase {
         const bool tune_shape = cfg.block_size <= 0 && cfg.ctas_per_sm <= 0 && cfg.use_graph <= 0 && !mode;
         int cur_shape = tune_shape ? (shape_sel >= 0 ? shape_sel : 0) : 0;
         CK(shape(cur_shape));
+        std::vector<uint2> div;   // (lives until ws has copied it)
         Params<Real> P;
         std::memset(&P, 0, sizeof(P));
         P.T = T; P.G = G;
@@ -2805,13 +2825,13 @@ struct Engine : EngineBase {
             P.pslot = (const uint2 *)d_pslot.p;
             P.nprob = nprob;
             if (group > 1) {
-                std::vector<uint2> div(nprob);
+                div.resize(nprob);
                 for (int k = 0; k < nprob; ++k) {
                     int l;
                     fast_divisor((uint32_t)std::max<long long>(1, phist[k] / nbatch), div[k].x, l);
                     div[k].y = (unsigned)l;
                 }
-                CK(cudaMemcpy(d_pslot.p, div.data(), nprob * sizeof(uint2), cudaMemcpyHostToDevice));
+                CK(cudaMemcpyAsync(d_pslot.p, div.data(), nprob * sizeof(uint2), cudaMemcpyHostToDevice, ws));
             }
             P.slot_last = group - 1;
         }
@@ -2829,8 +2849,6 @@ struct Engine : EngineBase {
         if (use_loop) build_loop_graph(P, gp, ge, bs, Multi, hfl);
         const bool looping = use_loop && gexec_loop;
         unsigned *counts = (unsigned *)d_counts.p;
-        CK(cudaEventRecord(ev_in, st));
-        CK(cudaStreamWaitEvent(ws, ev_in, 0));
         CK(set_caps(ws));
         std::vector<long long> hprefix(nprob + 1), hfirst(nprob + 1);
         for (int b = 0; b < nbatch; b += group) {
@@ -3106,7 +3124,7 @@ struct Engine : EngineBase {
         CK(cudaMemset(d_dose.p, 0, nvox * sizeof(double)));
         CK(cudaMemset(d_sum.p, 0, nvox * sizeof(double)));
         CK(cudaMemset(d_sum2.p, 0, nvox * sizeof(double)));
-        return 0;
+        return uploaded(err);
     }
 
     // Each call transports the next histories of every phantom: the first
@@ -3172,6 +3190,7 @@ struct Engine : EngineBase {
         P.requeue_lanes = 0;
         P.inter_batch = cfg.inter_batch > 0 ? std::min(cfg.inter_batch, 32) : (cfg.inter_batch < 0 ? 1 : 8);
         P.inter_batch_p = cfg.inter_batch > 0 ? std::min(cfg.inter_batch, 32) : (cfg.inter_batch < 0 ? 1 : 12);
+        CK(wait_uploads(st));
         // the array keeps the previous call's contents: clear the counters
         CK(cudaMemsetAsync(scratch, 0, 1024, st));
         CK(set_caps(st));
@@ -3475,7 +3494,7 @@ int egsgpu_set_source(egsgpu_handle *h, const egsgpu_source *s) {
     }
     h->S = S;
     h->have_source = true;
-    return 0;
+    return h->eng->uploaded(h->err);
 }
 
 int egsgpu_run(egsgpu_handle *h, long long first, long long n, int n_batch, uint32_t seed, void *stream) {
