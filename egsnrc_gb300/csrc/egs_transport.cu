@@ -1971,7 +1971,7 @@ struct EngineBase {
     virtual int run_noalloc(const Source &S, long long first, long long n, uint32_t seed, double *dose,
                             cudaStream_t st, unsigned char *scratch, size_t scratch_bytes, std::string &err) = 0;
     virtual int problems(int n, const PhantomDesc *pd, const Source *src, std::string &err) = 0;
-    virtual int uploaded(std::string &err) = 0;   // after uploads made by the caller: runs wait for them
+    virtual int source_set(std::string &err) = 0;   // another source: runs wait for its upload
     virtual int run_multi(const Source &Smax, int nbatch, cudaStream_t st, std::string &err) = 0;
     virtual int adjoint(const Source &S, long long first, long long n, uint32_t seed, const double *w, double *grad,
                         std::string &err) = 0;
@@ -2107,10 +2107,14 @@ struct Engine : EngineBase {
     // or a non-blocking stream of the caller).  Every call that uploads or clears
     // records this event behind its work, and every run waits for it on the device.
     cudaEvent_t ev_up = nullptr;
-    int uploaded(std::string &err) override {
+    int uploaded(std::string &err) {
         if (!ev_up) CK(cudaEventCreateWithFlags(&ev_up, cudaEventDisableTiming));
         CK(cudaEventRecord(ev_up, cudaStreamLegacy));
         return 0;
+    }
+    int source_set(std::string &err) override {
+        group_most = NO_LIMIT;
+        return uploaded(err);
     }
     cudaError_t wait_uploads(cudaStream_t st) { return ev_up ? cudaStreamWaitEvent(st, ev_up, 0) : cudaSuccess; }
 
@@ -2404,6 +2408,7 @@ struct Engine : EngineBase {
     int geometry(int nx, int ny, int nz, const double *xb, const double *yb, const double *zb, const int32_t *med,
                  const double *rhor, std::string &err) override {
         nprob = 0;
+        group_most = NO_LIMIT;
         nvox = (long long)nx * ny * nz;
         std::atomic<bool> mixed{false};
         host_parallel(nvox, [&](long long b, long long e) {
@@ -2670,9 +2675,14 @@ struct Engine : EngineBase {
     // wavefronts, each into a tally slot of its own.  Every wavefront ends in a
     // tail as long as its longest history (several ms: a charged particle's
     // steps follow one another), so batches smaller than a wavefront are
-    // grouped until they fill one: `most` histories, a wavefront that the queues
-    // hold by the estimate the chunk autotuner starts from.  A batch that fills
-    // a wavefront by itself keeps its own.  The slots take at most 2 GiB.
+    // grouped until they fill one: `most` histories, the present chunk or what the
+    // queues hold by the estimate the chunk autotuner starts from.  A batch that
+    // fills a wavefront by itself keeps its own.  The slots take at most 2 GiB.
+    // `most` is no promise: the chunk may come from another source or phantom on
+    // the same handle, and the estimate has a floor.  A group that overflows the
+    // queues is undone (mark_group) and runs again in chunks of the estimate, and
+    // then its batches one at a time, so that a run fails only where a batch by
+    // itself does not fit.
     // One GB300, 10 batches one at a time -> grouped: water30 1e4 histories
     // 52.7 -> 7.1 ms, slab64 2e6 98.7 -> 22.7 ms, 2e5 20 MeV electrons in
     // 128^3 voxels 814 -> 164 ms.
@@ -2703,6 +2713,36 @@ struct Engine : EngineBase {
         }
         CK(cudaMemsetAsync((char *)d_dose.p + one * dose_slots, 0, one * (slots - dose_slots), ws));
         dose_slots = slots;
+        return 0;
+    }
+
+    // Largest group (histories) after one that did not fit the queues: half of it,
+    // until the source or the phantom changes.
+    static constexpr long long NO_LIMIT = 1LL << 62;
+    long long group_most = NO_LIMIT;
+    DevMem d_mark, d_mark_hist;
+    static constexpr size_t MARK_EN = 2 * sizeof(double), MARK_CN = CNT_N * sizeof(unsigned long long),
+                            MARK_ER = 2 * sizeof(int);
+    bool mark_room() {
+        if (d_mark.alloc(MARK_EN + MARK_CN + MARK_ER) == cudaSuccess &&
+            (hist_n <= 0 || d_mark_hist.alloc(hist_n * sizeof(double)) == cudaSuccess)) return true;
+        cudaGetLastError();
+        return false;
+    }
+    // What a group's wavefronts add to besides its slots (energy, counters, error
+    // flags and the per-history tally): copied aside in front of the group, and
+    // back with its slots cleared where it has to be undone.
+    int mark_group(bool back, int slots, std::string &err) {
+        const size_t en = MARK_EN, cn = MARK_CN, er = MARK_ER, hn = hist_n > 0 ? hist_n * sizeof(double) : 0;
+        char *m = (char *)d_mark.p;
+        auto copy = [&](void *own, void *mark, size_t n) {
+            return cudaMemcpyAsync(back ? own : mark, back ? mark : own, n, cudaMemcpyDeviceToDevice, ws);
+        };
+        CK(copy(d_energy.p, m, en));
+        CK(copy(d_counters.p, m + en, cn));
+        CK(copy(d_error.p, m + en + cn, er));
+        if (hn) CK(copy(d_hist.p, d_mark_hist.p, hn));
+        if (back) CK(cudaMemsetAsync(d_dose.p, 0, (size_t)nvox * slots * sizeof(double), ws));
         return 0;
     }
 
@@ -2740,7 +2780,7 @@ struct Engine : EngineBase {
             total = 0;
             for (long long c : phist) total += c;
         }
-        int group = mode ? 1 : batches_per_group(total, nbatch, tune ? chunk : std::min(chunk, chunk0));
+        int group = mode ? 1 : batches_per_group(total, nbatch, std::min(tune ? chunk : std::min(chunk, chunk0), group_most));
         if (cfg.use_graph > 0 && group < nbatch) group = 1;
         // persistent grids, one per kernel: never more CTAs than can be
         // resident at once (the photon kernel, with fewer registers, fits more
@@ -2759,6 +2799,8 @@ struct Engine : EngineBase {
         CK(cudaEventRecord(ev_in, st));
         CK(cudaStreamWaitEvent(ws, ev_in, 0));
         CK(wait_uploads(ws));
+        const bool can_undo = !mode && mark_room();
+        if (!can_undo) group = 1;
         if (int rc = ensure_slots(group, err)) return rc;
         // The launch shape of candidate k (see SHAPES): threads per CTA and the
         // grids of both kernels.
@@ -2843,16 +2885,21 @@ struct Engine : EngineBase {
         }
         P.pin = q[0]; P.ein = q[2]; P.pout = q[0]; P.eout = q[2];
         const bool use_graph = cfg.use_graph == 1 && graph_ok && !mode;
-        if (use_graph) build_graph(P, gp, ge, bs, Multi, hfl);
-        const bool graph = use_graph && gexec;
         const bool use_loop = cfg.use_graph == 2 && loop_ok && !mode;
-        if (use_loop) build_loop_graph(P, gp, ge, bs, Multi, hfl);
-        const bool looping = use_loop && gexec_loop;
+        bool graph = false, looping = false;
+        auto record = [&] {   // the graphs hold P, its slot parameters among it
+            if (use_graph) build_graph(P, gp, ge, bs, Multi, hfl);
+            if (use_loop) build_loop_graph(P, gp, ge, bs, Multi, hfl);
+            graph = use_graph && gexec;
+            looping = use_loop && gexec_loop;
+        };
+        record();
         unsigned *counts = (unsigned *)d_counts.p;
         CK(set_caps(ws));
         std::vector<long long> hprefix(nprob + 1), hfirst(nprob + 1);
-        for (int b = 0; b < nbatch; b += group) {
-            const int nb = std::min(group, nbatch - b);   // batches [b, b + nb) run together
+        bool grow = true;   // not after an undone group: its second try keeps the chunk it starts with
+        for (int b = 0, nb; b < nbatch; b += nb) {
+            nb = std::min(group, nbatch - b);   // batches [b, b + nb) run together
             long long b0, bn;
             // the histories of batches [b, b + nb) of a run of cnt from f0
             auto group_range = [&](long long f0, long long cnt, long long &f, long long &c) {
@@ -2882,6 +2929,10 @@ struct Engine : EngineBase {
                 P.slot_last = nb - 1;
                 if (!Multi) P.slot_first = (unsigned)b0;
             }
+            const bool marked = can_undo && (nb > 1 || (tune && chunk > chunk0));
+            if (marked)
+                if (int rc = mark_group(false, 0, err)) return rc;
+            bool over = false;   // a queue was too short
             for (long long c0 = b0, cn = 0; c0 < b0 + bn; c0 += cn) {
                 cn = std::min(chunk, b0 + bn - c0);   // the autotuner may change `chunk` below
                 // shapes are timed on chunks of one size: full chunks once the
@@ -2911,13 +2962,10 @@ struct Engine : EngineBase {
                     CK(cudaStreamSynchronize(ws));
                     prof_ms[0] += elapsed(ev[0], ev[1]); ++prof_n[0];
                     prof_n[1] += nr; prof_n[2] += nr;
-                    if (h[8] > capacity || h[0] > capacity || h[4] > capacity) {
-                        err = "particle queue capacity exceeded; lower egsgpu_config.chunk or raise capacity";
-                        return EGSGPU_ERR_CAPACITY;
-                    }
+                    over = h[8] > capacity || h[0] > capacity || h[4] > capacity;
                     done = (h[0] == 0 && h[4] == 0);
                 }
-                for (int rep = 0; rep < 100000 / ROUNDS && !done && !looping; ++rep) {
+                for (int rep = 0; rep < 100000 / ROUNDS && !done && !over && !looping; ++rep) {
                     if (graph) CK(cudaGraphLaunch(gexec, ws));
                     else CK(enqueue_rounds(P, gp, ge, bs, true, Multi, adj, hfl));
                     CK(cudaMemcpyAsync(h, counts, sizeof(h), cudaMemcpyDeviceToHost, ws));
@@ -2931,13 +2979,16 @@ struct Engine : EngineBase {
                         ++prof_n[1];
                         ++prof_n[2];
                     }
-                    if (h[8] > capacity || h[0] > capacity || h[4] > capacity) {
-                        err = "particle queue capacity exceeded; lower egsgpu_config.chunk or raise capacity";
-                        return EGSGPU_ERR_CAPACITY;
-                    }
+                    over = h[8] > capacity || h[0] > capacity || h[4] > capacity;
                     done = (h[0] == 0 && h[4] == 0);
                 }
-                if (!done) { err = "wavefront did not drain"; return EGSGPU_ERR_LOOP; }
+                if (over) break;
+                if (!done) {
+                    if (marked)   // (no deposits stay in the slots)
+                        if (int rc = mark_group(true, nb, err)) return rc;
+                    err = "wavefront did not drain";
+                    return EGSGPU_ERR_LOOP;
+                }
                 if (trying) {
                     const double dt = std::chrono::duration<double>(std::chrono::steady_clock::now() - t_chunk).count();
                     shape_rate[shape_try] = cn / std::max(dt, 1e-9);
@@ -2961,7 +3012,7 @@ struct Engine : EngineBase {
                     if (peak > 2 * (capacity / 3)) {
                         tuned_chunk = chunk = std::max<long long>(1024, chunk / 2);
                         tune_done = true;
-                    } else if (!tune_done) {
+                    } else if (!tune_done && grow) {
                         if (best_rate > 0 && rate < 0.9 * best_rate) {
                             tuned_chunk = chunk = best_chunk;
                             tune_done = true;
@@ -2972,6 +3023,26 @@ struct Engine : EngineBase {
                         }
                     }
                 }
+            }
+            if (over) {   // the group again, in smaller wavefronts where that is left to do
+                if (!marked) {
+                    err = "particle queue capacity exceeded; lower egsgpu_config.chunk or raise capacity";
+                    return EGSGPU_ERR_CAPACITY;
+                }
+                if (int rc = mark_group(true, nb, err)) return rc;
+                if (tune && chunk > chunk0) {   // a chunk tuned on other particles: the tuner starts over
+                    tuned_chunk = chunk = chunk0;
+                    best_rate = 0;
+                    tune_done = false;
+                    grow = false;
+                } else {                        // this group's batches, and the rest, one at a time
+                    group_most = bn / 2;
+                    group = 1;
+                    P.slot_last = 0;
+                    record();
+                }
+                nb = 0;
+                continue;
             }
             if (mode) { CK(cudaStreamSynchronize(ws)); continue; }
             CK(cudaEventRecord(ev[6], ws));
@@ -3115,6 +3186,7 @@ struct Engine : EngineBase {
         G = gs[0];
         nvox = tot;
         nprob = n;
+        group_most = NO_LIMIT;
         homogeneous = false;
         pdone.assign(n, 0);
         dose_slots = 1;
@@ -3494,7 +3566,7 @@ int egsgpu_set_source(egsgpu_handle *h, const egsgpu_source *s) {
     }
     h->S = S;
     h->have_source = true;
-    return h->eng->uploaded(h->err);
+    return h->eng->source_set(h->err);
 }
 
 int egsgpu_run(egsgpu_handle *h, long long first, long long n, int n_batch, uint32_t seed, void *stream) {
