@@ -2677,7 +2677,8 @@ struct Engine : EngineBase {
     // steps follow one another), so batches smaller than a wavefront are
     // grouped until they fill one: `most` histories, the present chunk or what the
     // queues hold by the estimate the chunk autotuner starts from.  A batch that
-    // fills a wavefront by itself keeps its own.  The slots take at most 2 GiB.
+    // fills a wavefront by itself keeps its own.  The slots take at most 2 GiB, and
+    // at most a sixth of the free memory (ensure_slots).
     // `most` is no promise: the chunk may come from another source or phantom on
     // the same handle, and the estimate has a floor.  A group that overflows the
     // queues is undone (mark_group) and runs again in chunks of the estimate, and
@@ -2700,8 +2701,12 @@ struct Engine : EngineBase {
         if (slots <= dose_slots) return 0;
         const size_t one = (size_t)nvox * sizeof(double), had = d_dose.n / one;
         if ((size_t)slots > had) {
+            // at most a sixth of the free memory, as the queues (default_capacity): the
+            // rest is for others, and for kernels whose stacks the driver places at
+            // their first launch (the adjoint's take 2 GB); else one batch at a time
+            size_t fr = 0, tot = 0;
             DevMem more;
-            if (more.alloc(one * slots) != cudaSuccess) {   // not enough memory: one batch at a time
+            if (cudaMemGetInfo(&fr, &tot) != cudaSuccess || one * slots > fr / 6 || more.alloc(one * slots) != cudaSuccess) {
                 cudaGetLastError();
                 slots = 1;
                 return 0;

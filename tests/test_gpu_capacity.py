@@ -100,3 +100,30 @@ def test_a_batch_too_large_by_itself_is_refused_and_leaves_the_handle_usable():
     big = engine()
     big.set_source(photons(6.0))
     agree(results(e, 300, 10, 5), results(big, 300, 10, 5))
+
+
+def test_batch_slots_leave_a_nearly_full_device_its_memory():
+    """With 3 GiB free the slots of ten batches (1.1 GB at 240^3 voxels) are not
+    taken: batches run one at a time, with the same result."""
+    import torch
+    g = W.centred_geometry(240, 0.125)
+    out = []
+    for fill in (False, True):
+        e = eg.DoseEngine([W.WATER], ecut=0.7, pcut=0.01, precision=64, capacity=1 << 16)
+        e.set_geometry(g)
+        e.set_source(photons(2.0))
+        e.run(100, nbatch=1, seed=2)     # queues and kernels are in place
+        e.reset()
+        torch.cuda.synchronize()
+        keep = torch.empty(torch.cuda.mem_get_info()[0] - (3 << 30), dtype=torch.uint8, device="cuda") if fill else None
+        free = torch.cuda.mem_get_info()[0]
+        e.run(4000, nbatch=20, seed=2)
+        torch.cuda.synchronize()
+        taken = free - torch.cuda.mem_get_info()[0]
+        del keep
+        torch.cuda.empty_cache()
+        if fill:
+            assert taken <= free // 6 + (64 << 20)
+        out.append(e.tallies()[:2])
+        e.close()
+    agree(out[1], out[0])
