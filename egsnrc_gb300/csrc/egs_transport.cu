@@ -2122,9 +2122,7 @@ struct Engine : EngineBase {
         CK(cudaMemset(d_dose.p, 0, nv * dose_slots * sizeof(double)));
         CK(cudaMemset(d_sum.p, 0, nv * sizeof(double)));
         CK(cudaMemset(d_sum2.p, 0, nv * sizeof(double)));
-        CK(cudaMemset(d_energy.p, 0, 2 * sizeof(double)));
-        CK(cudaMemset(d_counters.p, 0, CNT_N * sizeof(unsigned long long)));
-        CK(cudaMemset(d_error.p, 0, 2 * sizeof(int)));
+        CK(cudaMemset(d_energy.p, 0, TOTALS));
         for (int k = 0; k < 4; ++k) { prof_ms[k] = 0; prof_n[k] = 0; }
         return uploaded(err);
     }
@@ -2220,7 +2218,9 @@ struct Engine : EngineBase {
     DevMem d_counts;   // 4 queues x (count, head)
     unsigned capacity = 0;
     // tallies
-    DevMem d_dose, d_sum, d_sum2, d_energy, d_counters, d_error, d_hist;
+    DevMem d_dose, d_sum, d_sum2, d_energy, d_hist;
+    struct Part { void *p = nullptr; } d_counters, d_error;   // behind d_energy, cleared and marked with it
+    static constexpr size_t TOTALS = 2 * sizeof(double) + CNT_N * sizeof(unsigned long long) + 2 * sizeof(int);
     int dose_slots = 1;   // batch slots of d_dose in use (all zero between runs)
     long long hist_first = 0, hist_n = 0;
     int sm_count = 0;
@@ -2371,12 +2371,10 @@ struct Engine : EngineBase {
         T.nmed = nmed;
         T.ecut = (Real)ecut; T.pcut = (Real)pcut; T.skindepth = (Real)skindepth; T.smaxir = (Real)smax;
         // tallies that do not depend on the geometry
-        CK(d_energy.alloc(2 * sizeof(double)));
-        CK(d_counters.alloc(CNT_N * sizeof(unsigned long long)));
-        CK(d_error.alloc(2 * sizeof(int)));
-        CK(cudaMemset(d_energy.p, 0, 2 * sizeof(double)));
-        CK(cudaMemset(d_counters.p, 0, CNT_N * sizeof(unsigned long long)));
-        CK(cudaMemset(d_error.p, 0, 2 * sizeof(int)));
+        CK(d_energy.alloc(TOTALS));
+        d_counters.p = (double *)d_energy.p + 2;
+        d_error.p = (unsigned long long *)d_counters.p + CNT_N;
+        CK(cudaMemset(d_energy.p, 0, TOTALS));
         return uploaded(err);
     }
 
@@ -2726,10 +2724,8 @@ struct Engine : EngineBase {
     static constexpr long long NO_LIMIT = 1LL << 62;
     long long group_most = NO_LIMIT;
     DevMem d_mark, d_mark_hist;
-    static constexpr size_t MARK_EN = 2 * sizeof(double), MARK_CN = CNT_N * sizeof(unsigned long long),
-                            MARK_ER = 2 * sizeof(int);
     bool mark_room() {
-        if (d_mark.alloc(MARK_EN + MARK_CN + MARK_ER) == cudaSuccess &&
+        if (d_mark.alloc(TOTALS) == cudaSuccess &&
             (hist_n <= 0 || d_mark_hist.alloc(hist_n * sizeof(double)) == cudaSuccess)) return true;
         cudaGetLastError();
         return false;
@@ -2738,15 +2734,11 @@ struct Engine : EngineBase {
     // flags and the per-history tally): copied aside in front of the group, and
     // back with its slots cleared where it has to be undone.
     int mark_group(bool back, int slots, std::string &err) {
-        const size_t en = MARK_EN, cn = MARK_CN, er = MARK_ER, hn = hist_n > 0 ? hist_n * sizeof(double) : 0;
-        char *m = (char *)d_mark.p;
         auto copy = [&](void *own, void *mark, size_t n) {
             return cudaMemcpyAsync(back ? own : mark, back ? mark : own, n, cudaMemcpyDeviceToDevice, ws);
         };
-        CK(copy(d_energy.p, m, en));
-        CK(copy(d_counters.p, m + en, cn));
-        CK(copy(d_error.p, m + en + cn, er));
-        if (hn) CK(copy(d_hist.p, d_mark_hist.p, hn));
+        CK(copy(d_energy.p, d_mark.p, TOTALS));
+        if (hist_n > 0) CK(copy(d_hist.p, d_mark_hist.p, hist_n * sizeof(double)));
         if (back) CK(cudaMemsetAsync(d_dose.p, 0, (size_t)nvox * slots * sizeof(double), ws));
         return 0;
     }
