@@ -162,7 +162,8 @@ static __host__ __device__ __noinline__ uint4 philox_block(uint32_t b, uint32_t 
 
 // The generator keeps a window of the stream's next W numbers (W / 4 Philox
 // blocks; number i in word i & (W - 1); `lim` is one past the highest held).  A
-// draw computes only a block that is missing.  The transport loops call
+// checked draw (u, u2) computes a block that is missing; get and get2 compute
+// none and rely on what ahead or ensure made present.  The transport loops call
 // ahead(k) where the warp is converged, so that the blocks the lanes will
 // need for the coming step are computed there, by all lanes together, instead
 // of at whichever draw site a lane's counter happens to cross into a new block
@@ -173,7 +174,8 @@ static __host__ __device__ __noinline__ uint4 philox_block(uint32_t b, uint32_t 
 // particle copies stay small and a copy never reads blocks it did not compute.
 //
 // The window belongs to the thread: on the device it is a column of a shared
-// array (word w of thread t at [w][t], free of bank conflicts; 8 KB per CTA),
+// array (word w of thread t at [w][t], free of bank conflicts; W * 512 B per CTA:
+// 8 KB in the photon kernel, 16 KB in the electron kernel),
 // which leaves position, key and limit in registers and makes a draw one
 // shared-memory load, inlined.  With the window in local memory (RngLocal) the
 // whole particle lives there too, around every out-of-line draw.  Local -> shared
@@ -236,7 +238,7 @@ struct RngW {
     // A draw that checks costs more than its check: the lanes that take its slow
     // path leave the others, and the code behind it runs once for each group.  With
     // one check for a pair, none in the step's straight-line draws and no integer
-    // conversion, one GB300: slab64 1e8 409 -> 363 ms, water30 1e6 23.4 -> 20.0 ms,
+    // conversion, one GB300, warm L2: slab64 1e8 409 -> 363 ms, water30 1e6 23.4 -> 20.0 ms,
     // water128e 2e5 114 -> 101 ms, perturbed64 32.1 -> 28.7 ms, noalloc 512 1.46 ->
     // 1.38 ms.
     __host__ __device__ inline float get() {
@@ -313,12 +315,12 @@ struct RngLocal {
         }
         if (b > next) next = b;
     }
-    // Out of line (as is azimuth): the electron step loop is larger than the
-    // instruction caches, and one shared copy of the draw for its ~30 call
-    // sites measured 20-40% faster than inlined copies, even though the
-    // generator state then lives in local memory around each call.  Sites that
-    // take two numbers in a row call u2 (one call instead of two: +3% on
-    // electron-dominated phantoms).
+    // Out of line (as is the azimuth of this class), for what still draws
+    // through it, the precision split's electron step above all: with the state in
+    // local memory an inlined draw is long, and one shared copy for the ~30 call
+    // sites of a step loop measured 20-40% faster than inlined copies.  (RngW's
+    // draw is a shared-memory load and is inlined.)  Sites that take two numbers in
+    // a row call u2 (one call instead of two: +3% on electron-dominated phantoms).
     __host__ __device__ __noinline__ float u() { return draw(); }
     __host__ __device__ __noinline__ float2 u2() {
         float a = draw();

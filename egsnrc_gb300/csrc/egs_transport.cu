@@ -286,8 +286,8 @@ __device__ inline void q_load(const Queue<Real> &q, unsigned i, uint32_t seed, P
 // every warp the same number k of them (the lowest k lanes) and fetches no
 // more.  Filling whole warps instead leaves most warps of the grid empty and
 // makes each track wait, step by step, for the divergent paths of 31 others;
-// the longest track is what such a launch takes (512 slab64 histories: 2.85 ->
-// 1.71 ms, 1e4 water30 histories: 6.6 -> 4.6 ms).  Returns the warp's first
+// the longest track is what such a launch takes (repeated calls with a warm L2: 512
+// slab64 histories 2.85 -> 1.71 ms, 1e4 water30 histories 6.6 -> 4.6 ms).  Returns the warp's first
 // record.  The fetch in front of the loop is a copy of its own: a branch at the
 // fetch inside the loop cost dense launches 3%.  Not with requeue_lanes, which
 // would park such thin warps again before they took a step.
@@ -924,8 +924,9 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(Real) == 4 ? 8 : 1) k_photon
         // to its faces are computed.  The walk is two thirds of this kernel's time
         // and bound by its dependent chain and by issue; decoding the index, choosing
         // the planes and waiting for the medium at every voxel cost 30% of it
-        // (one GB300: slab64 1e8 histories 488 -> 444 ms, 2e6 18.3 -> 17.2 ms, 512
-        // noalloc 1.54 -> 1.48 ms).
+        // (one GB300, warm L2: slab64 1e8 histories 488 -> 444 ms, 2e6 18.3 -> 17.2 ms,
+        // 512 noalloc 1.54 -> 1.48 ms).  egsgpu_geometry_query does not run this walk;
+        // it is held to the oracle's by the history-by-history FP64 comparisons.
         const Geom<Real> &GP = geom_of<Real, Multi>(P, p.pb);
         const Real *xb = GP.xb, *yb = GP.yb, *zb = GP.zb;
         int jx, jy, jz;
@@ -1173,9 +1174,10 @@ __device__ __noinline__ Real wide_eloss(const Tables<Real> &T, const MedScalars<
 // meet again after the start of a new step sequence, before the face distances
 // and after the deflection: left alone, the compiler threads the new sequences
 // past the join, and the warp ran the whole step 1.2-1.4 times per iteration in
-// two thin groups.  FP32: five CTAs per SM, the most at which nothing spills
-// (94-96 registers; six were 80 with spills).  Both together, one GB300:
-// slab64 1e8 histories 526 -> 500 ms, water128e 2e5 163 -> 156 ms, perturbed64
+// two thin groups.  FP32: five CTAs per SM (96 registers, 32 B of spill stores a
+// thread; with several phantoms 66 B, PRESTA-I 54 B), where six have 80 registers
+// and spill the particle.  Both together, when five spilled nothing yet (the
+// shared generator window came later), one GB300: slab64 1e8 histories 526 -> 500 ms, water128e 2e5 163 -> 156 ms, perturbed64
 // 46.0 -> 40.8 ms.  HOWFARLESS and the precision split keep six CTAs and only the
 // join before the deflection: measured no faster otherwise (HOWFARLESS 1e6 at
 // five 87.5 against 86.5 ms).

@@ -171,7 +171,11 @@ int egsgpu_set_source(egsgpu_handle *h, const egsgpu_source *src);
  * Philox streams keyed by (seed, history index); results are independent
  * of chunking. Accumulates into the handle's tallies (call egsgpu_reset to
  * clear). `stream` is a cudaStream_t or NULL for the default stream; the
- * call returns after the work on it has completed.
+ * call returns after the work on it has completed.  The run also waits for
+ * the uploads and the clearing of earlier calls on this handle, so a
+ * non-blocking stream is fine.  EGSGPU_ERR_CAPACITY means that a batch by
+ * itself does not fit the queues (or a chunk that the caller has set): batches
+ * transported together that do not fit are run again in smaller wavefronts.
  * Replaces EGS_Application::runSimulation / simulateSingleShower / egsShower
  * (egs++/egs_application.cpp:839-959, interface/egs_interface2.c:92-99). */
 int egsgpu_run(egsgpu_handle *h, long long first, long long n, int n_batch, uint32_t seed,
@@ -251,8 +255,10 @@ int egsgpu_set_history_tally(egsgpu_handle *h, long long first, long long n);
 int egsgpu_get_history_tally(egsgpu_handle *h, double *out);
 
 /* Geometry queries on the handle's phantom (set by egsgpu_set_xyz_geometry),
- * computed on the GPU by the transport kernels' own geometry functions in the
- * handle's precision.  A checking aid: each op is the EGS_XYZGeometry method
+ * computed on the GPU by the engine's geometry functions in the handle's
+ * precision: those of the electron steps and of the source (the photon kernel
+ * walks voxels with the same arithmetic in code of its own).  A checking aid:
+ * each op is the EGS_XYZGeometry method
  * it replaces (egs++/geometry/egs_nd_geometry/egs_nd_geometry.h):
  *   op 0  isWhere (:791-805): inew[i] = region of point x[3i..3i+2], -1 outside;
  *   op 1  howfar (:963-1104), or howfarFromOut (:1281-1379) when ireg[i] < 0:
