@@ -1973,7 +1973,7 @@ struct EngineBase {
     virtual int run_noalloc(const Source &S, long long first, long long n, uint32_t seed, double *dose,
                             cudaStream_t st, unsigned char *scratch, size_t scratch_bytes, std::string &err) = 0;
     virtual int problems(int n, const PhantomDesc *pd, const Source *src, std::string &err) = 0;
-    virtual int source_set(std::string &err) = 0;   // another source: runs wait for its upload
+    virtual int source_set(bool upload, std::string &err) = 0;   // another source; runs wait for its upload, if any
     virtual int run_multi(const Source &Smax, int nbatch, cudaStream_t st, std::string &err) = 0;
     virtual int adjoint(const Source &S, long long first, long long n, uint32_t seed, const double *w, double *grad,
                         std::string &err) = 0;
@@ -2114,9 +2114,9 @@ struct Engine : EngineBase {
         CK(cudaEventRecord(ev_up, cudaStreamLegacy));
         return 0;
     }
-    int source_set(std::string &err) override {
+    int source_set(bool upload, std::string &err) override {
         group_most = NO_LIMIT;
-        return uploaded(err);
+        return upload ? uploaded(err) : 0;   // (no work on the default stream without need)
     }
     cudaError_t wait_uploads(cudaStream_t st) { return ev_up ? cudaStreamWaitEvent(st, ev_up, 0) : cudaSuccess; }
 
@@ -2168,8 +2168,9 @@ struct Engine : EngineBase {
         if (n > 0) {
             CK(d_hist.alloc(n * sizeof(double)));
             CK(cudaMemset(d_hist.p, 0, n * sizeof(double)));
+            return uploaded(err);
         }
-        return uploaded(err);
+        return 0;
     }
     int read_history_tally(double *out, std::string &err) override {
         if (hist_n > 0) CK(cudaMemcpy(out, d_hist.p, hist_n * sizeof(double), cudaMemcpyDeviceToHost));
@@ -3565,7 +3566,7 @@ int egsgpu_set_source(egsgpu_handle *h, const egsgpu_source *s) {
     }
     h->S = S;
     h->have_source = true;
-    return h->eng->source_set(h->err);
+    return h->eng->source_set(s->shape == 2 || s->spectrum == 1, h->err);
 }
 
 int egsgpu_run(egsgpu_handle *h, long long first, long long n, int n_batch, uint32_t seed, void *stream) {
