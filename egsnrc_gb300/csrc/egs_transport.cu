@@ -287,10 +287,10 @@ __device__ inline void q_load(const Queue<Real> &q, unsigned i, uint32_t seed, P
 // more.  Filling whole warps instead leaves most warps of the grid empty and
 // makes each track wait, step by step, for the divergent paths of 31 others;
 // the longest track is what such a launch takes (repeated calls with a warm L2: 512
-// slab64 histories 2.85 -> 1.71 ms, 1e4 water30 histories 6.6 -> 4.6 ms).  Returns the warp's first
-// record.  The fetch in front of the loop is a copy of its own: a branch at the
-// fetch inside the loop cost dense launches 3%.  Not with requeue_lanes, which
-// would park such thin warps again before they took a step.
+// slab64 histories 2.85 -> 1.71 ms, 1e4 water30 histories 6.6 -> 4.6 ms).  Returns
+// the warp's first record.  The fetch in front of the loop is a copy of its own: a
+// branch at the fetch inside the loop cost dense launches 3%.  Not with
+// requeue_lanes, which would park such thin warps again before they took a step.
 __device__ inline unsigned sparse_share(unsigned nq, unsigned &k) {
     const unsigned per_cta = blockDim.x >> 5, nw = gridDim.x * per_cta;
     k = (nq + nw - 1) / nw;
@@ -1177,8 +1177,8 @@ __device__ __noinline__ Real wide_eloss(const Tables<Real> &T, const MedScalars<
 // two thin groups.  FP32: five CTAs per SM (96 registers, 32 B of spill stores a
 // thread; with several phantoms 66 B, PRESTA-I 54 B), where six have 80 registers
 // and spill the particle.  Both together, when five spilled nothing yet (the
-// shared generator window came later), one GB300: slab64 1e8 histories 526 -> 500 ms, water128e 2e5 163 -> 156 ms, perturbed64
-// 46.0 -> 40.8 ms.  HOWFARLESS and the precision split keep six CTAs and only the
+// shared generator window came later), one GB300: slab64 1e8 histories 526 -> 500
+// ms, water128e 2e5 163 -> 156 ms, perturbed64 46.0 -> 40.8 ms.  HOWFARLESS and the precision split keep six CTAs and only the
 // join before the deflection: measured no faster otherwise (HOWFARLESS 1e6 at
 // five 87.5 against 86.5 ms).
 template <class Real, bool Multi, bool Adj = false, bool HFL = false, bool PI = false, bool SPL = false>
@@ -2742,7 +2742,9 @@ struct Engine : EngineBase {
         };
         CK(copy(d_energy.p, d_mark.p, TOTALS));
         if (hist_n > 0) CK(copy(d_hist.p, d_mark_hist.p, hist_n * sizeof(double)));
-        if (back) CK(cudaMemsetAsync(d_dose.p, 0, (size_t)nvox * slots * sizeof(double), ws));
+        if (!back) return 0;
+        CK(cudaMemsetAsync(d_dose.p, 0, (size_t)nvox * slots * sizeof(double), ws));
+        CK(cudaStreamSynchronize(ws));   // the run may end here with an error: nothing stays in flight
         return 0;
     }
 
